@@ -285,6 +285,7 @@ int guarded(const char *what, F &&f) {
 }
 
 int plan_slot(int pattern, int sched) { return (pattern - 3) * 2 + sched; }
+constexpr int kProfileSlot = 7;  // the plan of gary_tc_features and gary_tc_profile: no hub rows
 
 PlanParams g_tuning;  // process-wide knobs of the counting plans (gary_tune)
 std::mutex g_tuning_mu;
@@ -395,8 +396,8 @@ extern "C" int gary_tc_features(gary_graph *g, float *d_x, uint8_t *d_legal, voi
   GARY_CHECK_ARG(g && d_x && d_legal, "NULL argument");
   return guarded("gary_tc_features", [&] {
     cudaStream_t s = gary::as_stream(stream);
-    const int slot = gary::plan_slot(GARY_PATTERN_TRIANGLE, GARY_SCHED_PLAIN);
-    if (!g->plans[slot]) GARY_TRY(gary::build_k3_plan(g, gary::tuned_params(), s, &g->plans[slot]));
+    const int slot = gary::kProfileSlot;
+    if (!g->plans[slot]) GARY_TRY(gary::build_k3_plan(g, gary::tuned_params(), s, &g->plans[slot], nullptr, false));
     return gary::k3_features(g, g->plans[slot], d_x, d_legal, s);
   });
 }
@@ -407,8 +408,8 @@ extern "C" int gary_tc_profile(gary_graph *g, int variant, uint64_t *d_cycles, u
   GARY_CHECK_ARG(variant >= -1 && variant <= 3, "variant must be -1 (plain) or 0..3");
   return guarded("gary_tc_profile", [&] {
     cudaStream_t s = gary::as_stream(stream);
-    const int slot = gary::plan_slot(GARY_PATTERN_TRIANGLE, GARY_SCHED_PLAIN);
-    if (!g->plans[slot]) GARY_TRY(gary::build_k3_plan(g, gary::tuned_params(), s, &g->plans[slot]));
+    const int slot = gary::kProfileSlot;
+    if (!g->plans[slot]) GARY_TRY(gary::build_k3_plan(g, gary::tuned_params(), s, &g->plans[slot], nullptr, false));
     gary::DevBuf<uint8_t> forced;
     if (variant >= 0) {
       GARY_TRY(forced.alloc(g->n, s));

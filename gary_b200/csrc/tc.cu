@@ -66,13 +66,16 @@ struct MinU64 {
   __host__ __device__ uint64_t operator()(uint64_t a, uint64_t b) const { return a < b ? a : b; }
 };
 
-// One candidate per padded word w of N+(u): the suffix after v = adj[w].
+// One candidate per padded word w of N+(u): the suffix after v = adj[w], up to
+// len[u] (null: the whole list); *cut += the suffix ids past len[u].
 // Words without a record get the key n - 1: in rank ids the top vertex has
 // no higher neighbour, so no record ever targets it, and the keys of an
 // n = 2^k graph fit k bits (one radix pass fewer than with the key n).
 __global__ void k_in_candidates(const uint2 *__restrict__ row, const uint32_t *__restrict__ adj,
                                 const uint32_t *__restrict__ rowid, uint64_t words, uint32_t n,
-                                uint32_t *__restrict__ keys, uint2 *__restrict__ vals) {
+                                const uint32_t *__restrict__ len, uint32_t *__restrict__ keys,
+                                uint2 *__restrict__ vals, unsigned long long *__restrict__ cut) {
+  unsigned long long mine = 0;
   for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < words;
        w += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t u = rowid[w];
@@ -84,12 +87,21 @@ __global__ void k_in_candidates(const uint2 *__restrict__ row, const uint32_t *_
       const uint32_t v = adj[w];
       const uint32_t rem = r.y - (uint32_t)pos - 1;
       if (rem && row[v].y) {
-        key = v;
-        val = make_uint2((uint32_t)(w + 1), rem);
+        const uint32_t end = len ? len[u] : r.y;
+        const uint32_t keep = end > (uint32_t)pos + 1 ? end - (uint32_t)pos - 1 : 0u;
+        mine += rem - keep;
+        if (keep) {
+          key = v;
+          val = make_uint2((uint32_t)(w + 1), keep);
+        }
       }
     }
     keys[w] = key;
     vals[w] = val;
+  }
+  if (len) {
+    mine = warp_sum_u64(mine);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(cut, mine);
   }
 }
 
@@ -306,7 +318,7 @@ __global__ void k_predict(const float *__restrict__ params, const float *__restr
 
 namespace {
 
-int build_in_index(gary_graph *g, cudaStream_t s, InIndex &in) {
+int build_in_index(gary_graph *g, cudaStream_t s, const DevBuf<uint32_t> &len, InIndex &in) {
   const uint32_t n = g->n;
   const uint64_t W = g->dag.words;
   if (W >= (1ull << 32)) {
@@ -317,13 +329,16 @@ int build_in_index(gary_graph *g, cudaStream_t s, InIndex &in) {
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
   DevBuf<uint32_t> keys, keys2;
   DevBuf<uint2> vals, vals2;
+  DevBuf<unsigned long long> cut;
+  GARY_TRY(cut.alloc(1, s));
   {
     DevBuf<uint32_t> rowid;
     GARY_TRY(padded_rowid(g->dag, rowid, s));
     GARY_TRY(keys.alloc(W, s));
     GARY_TRY(vals.alloc(W, s));
-    k_in_candidates<<<grid_for(W), kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, n, keys.p,
-                                                     vals.p);
+    GARY_CUDA(cudaMemsetAsync(cut.p, 0, 8, s));
+    k_in_candidates<<<grid_for(W), kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, n, len.p, keys.p,
+                                                     vals.p, cut.p);
     GARY_CUDA(cudaGetLastError());
   }
   GARY_TRY(keys2.alloc(W, s));
@@ -350,6 +365,7 @@ int build_in_index(gary_graph *g, cudaStream_t s, InIndex &in) {
     k_first_geq<<<1, 1, 0, s>>>(keys.p, W, n - 1, pos.p);
     GARY_CUDA(cudaGetLastError());
     GARY_CUDA(cudaMemcpyAsync(&m, pos.p, 8, cudaMemcpyDeviceToHost, s));
+    GARY_CUDA(cudaMemcpyAsync(&in.hub_work, cut.p, 8, cudaMemcpyDeviceToHost, s));
     GARY_CUDA(cudaStreamSynchronize(s));
   }
   in.records = m;
@@ -391,13 +407,18 @@ PlanParams resolve_params(PlanParams pp, uint64_t total_work) {
 }
 
 int build_k3_plan(gary_graph *g, const PlanParams &pp_in, cudaStream_t s, gary_count_plan **out,
-                  const float *model) {
+                  const float *model, bool hubs) {
   auto plan = std::make_unique<gary_count_plan>();
   const uint32_t n = g->n;
   ScratchAlloc pol_alloc{s};
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
   PhaseTrace tr("triangle plan", s);
-  GARY_TRY(build_in_index(g, s, plan->in));
+  {
+    DevBuf<uint32_t> len;
+    if (hubs) GARY_TRY(build_hub_rows(g, s, plan->hub, len));
+    tr.mark("hub rows");
+    GARY_TRY(build_in_index(g, s, len, plan->in));
+  }
   tr.mark("in-edge index");
   const PlanParams pp = resolve_params(pp_in, plan->in.total_work);
   plan->params = pp;
@@ -495,7 +516,8 @@ constexpr uint32_t kWarpBitmapSpan = bitmap_max_span(kWarpTableSlots);  // ids a
 // the chunk's octets, so short suffixes do not idle lanes.  Lists start on
 // 32-byte boundaries and are padded with kSentinel to a multiple of 8 words,
 // so an octet only ever holds words of its own list: ids up to and including
-// v before the suffix (all below min N+(v)) and padding.  Every set rejects
+// v before the suffix (all below min N+(v)) and padding (a suffix cut short by
+// hub rows ends with an octet).  Every set rejects
 // both as out of its [lo, lo + span] range, so no per-id mask is needed.
 // All 32 lanes must call.
 template <typename Set>
@@ -764,7 +786,7 @@ template <int WARPS, int MINB>
 __global__ void __launch_bounds__(WARPS * 32, MINB)
     k_tc_mid(GraphView g, const uint2 *__restrict__ inedge, const uint64_t *__restrict__ inptr,
              const uint32_t *__restrict__ light, const Tile *__restrict__ tiles, uint32_t n_cta,
-             TileRange rng, SchedState *sched, unsigned long long *__restrict__ out, VertexCtl ctl,
+             TileRange rng, HubView hub, SchedState *sched, unsigned long long *__restrict__ out, VertexCtl ctl,
              CtaSetCfg cfg) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ uint64_t bar;
@@ -796,26 +818,40 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
     }
   }
 
-  // phase 2: warp tiles, each warp on its own slots
+  // phase 2: warp tiles, each warp on its own slots, and hub rows.  Odd warps
+  // begin with the rows, even ones with the tiles, so that the rows' L2 reads
+  // and the tiles' shared-memory probes overlap on every SM.
   uint32_t *tab = smem + warp * kWarpTableSlots;
   const Tile *wt = tiles + n_cta;
-  while (alive) {
-    uint32_t t = 0;
-    if (lane == 0) t = rng.warp_lo + atomicAdd(&sched->next_warp, 1u);
-    t = __shfl_sync(kFull, t, 0);
-    if (t >= rng.warp_hi) break;
-    const Tile tl = wt[t];
-    if (tl.j1 != kGroupTile) {
-      cnt += warp_vertex(g, inedge, inptr, tl.v0, tl.j0, tl.j1, tab, lane, ctl);
+#pragma unroll 1
+  for (int part = 0; part < 2; ++part) {
+    if ((part ^ warp) & 1) {
+      while (alive && hub.lo < hub.hi) {
+        uint32_t i = 0;
+        if (lane == 0) i = hub.lo + atomicAdd(&sched->next_aux, 1u);
+        i = __shfl_sync(kFull, i, 0);
+        if (i >= hub.hi) break;
+        cnt += hub_vertex(g, hub, i, lane);
+      }
       continue;
     }
-    // a group of light vertices: list positions [v0, v1), 32 ids per load
-    for (uint32_t ib = tl.v0; ib < tl.v1; ib += 32) {
-      const uint32_t nb = min(32u, tl.v1 - ib);
-      const uint32_t myv = lane < nb ? light[ib + lane] : 0u;
-      for (uint32_t k = 0; k < nb; ++k)
-        cnt += warp_vertex(g, inedge, inptr, __shfl_sync(kFull, myv, k), 0, 0xFFFFFFFFu, tab, lane,
-                           ctl);
+    while (alive) {
+      uint32_t t = 0;
+      if (lane == 0) t = rng.warp_lo + atomicAdd(&sched->next_warp, 1u);
+      t = __shfl_sync(kFull, t, 0);
+      if (t >= rng.warp_hi) break;
+      const Tile tl = wt[t];
+      if (tl.j1 != kGroupTile) {
+        cnt += warp_vertex(g, inedge, inptr, tl.v0, tl.j0, tl.j1, tab, lane, ctl);
+        continue;
+      }
+      // a group of light vertices: list positions [v0, v1), 32 ids per load
+      for (uint32_t ib = tl.v0; ib < tl.v1; ib += 32) {
+        const uint32_t nb = min(32u, tl.v1 - ib);
+        const uint32_t myv = lane < nb ? light[ib + lane] : 0u;
+        for (uint32_t k = 0; k < nb; ++k)
+          cnt += warp_vertex(g, inedge, inptr, __shfl_sync(kFull, myv, k), 0, 0xFFFFFFFFu, tab, lane, ctl);
+      }
     }
   }
 
@@ -854,6 +890,8 @@ int launch_k3_impl(gary_graph *g, gary_count_plan *plan, unsigned long long *d_o
   if (!plan->span.p) GARY_TRY(plan->span.alloc_persistent(2 * kMaxCountCtas));
   ctl.span = plan->span.p;
   const TileRange rng = shard_range(plan->n_cta, plan->n_warp, shard, nshards);
+  auto part = [&](uint32_t k) { return (uint32_t)((uint64_t)plan->hub.n_list * k / nshards); };
+  const HubView hub{plan->hub.rows.p, plan->hub.rowof.p, plan->hub.list.p, plan->hub.cut.p, plan->hub.first, part(shard), part(shard + 1)};
   const uint32_t words = (uint32_t)(WARPS * kWarpTableSlots);
   const uint32_t cw = plan->params.cta_set_words;
   const CtaSetCfg cfg{cw && cw < words ? cw : words, plan->params.stage_polls};
@@ -865,13 +903,13 @@ int launch_k3_impl(gary_graph *g, gary_count_plan *plan, unsigned long long *d_o
   GARY_CUDA(cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), s));
   if (timed) GARY_CUDA(cudaEventRecord(g->ev0, s));
   kern<<<grid, WARPS * 32, smem, s>>>(g->view(), plan->in.inedge.p, plan->in.inptr.p, plan->light.p,
-                                      plan->tiles.p, plan->n_cta, rng, plan->sched.p, d_out, ctl, cfg);
+                                      plan->tiles.p, plan->n_cta, rng, hub, plan->sched.p, d_out, ctl, cfg);
   GARY_CUDA(cudaGetLastError());
   if (timed) GARY_CUDA(cudaEventRecord(g->ev1, s));
   g->last = gary_count_stats{};
   g->last.tiles = (rng.cta_hi - rng.cta_lo) + (rng.warp_hi - rng.warp_lo);
   g->last.cta_tiles = rng.cta_hi - rng.cta_lo;
-  g->last.work = plan->in.total_work;
+  g->last.work = plan->in.total_work + plan->in.hub_work;
   g->last_timed = timed;
   g->last_sched = plan->sched.p;
   g->last_span = plan->span.p;

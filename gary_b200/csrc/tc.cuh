@@ -4,6 +4,7 @@
 
 #include "bulk.cuh"
 #include "graph.cuh"
+#include "hub.cuh"
 #include "internal.cuh"
 
 namespace gary {
@@ -89,7 +90,7 @@ struct SchedState {
   uint32_t next_cta;
   uint32_t next_warp;
   uint32_t error;     // kLaunchErr* bits
-  uint32_t next_aux;  // a third queue (the 4-cycle kernel's medium vertices)
+  uint32_t next_aux;  // a third queue (counted hub-row vertices; the 4-cycle kernel's medium vertices)
   uint32_t cta_path[4];  // triangle CTA tiles by the set that held N+(v) (kPath*)
   uint32_t next_big;     // a fourth queue (4-clique vertices whose rows fit shared memory)
 };
@@ -100,6 +101,7 @@ enum : uint32_t { kPathBitmap = 0, kPathBuckets = 1, kPathStaged = 2, kPathSampl
 // In-edge index of the middle-vertex formulation.  For every oriented edge
 // u -> v whose list suffix after v is non-empty, and with d+(v) > 0:
 //   inedge[k] = {first word of N+(u) after v, length of that suffix}
+// (the suffix ends at u's first hub neighbour when u is counted by hub rows)
 // grouped by v: v's records are inedge[inptr[v] .. inptr[v+1]).
 struct InIndex {
   DevBuf<uint2> inedge;
@@ -107,6 +109,7 @@ struct InIndex {
   DevBuf<uint64_t> work;  // per v: sum of suffix lengths (probes)
   uint64_t records = 0;
   uint64_t total_work = 0;
+  uint64_t hub_work = 0;  // suffix ids the hub rows count instead
 };
 
 }  // namespace gary
@@ -114,6 +117,7 @@ struct InIndex {
 struct gary_count_plan {
   gary::PlanParams params;
   gary::InIndex in;
+  gary::HubRows hub;
   gary::DevBuf<uint8_t> vclass;
   gary::DevBuf<uint32_t> light;  // light vertices (group tiles index this list)
   uint32_t n_light = 0;
@@ -128,9 +132,11 @@ struct gary_count_plan {
 };
 
 namespace gary {
-// model: host copy of a cost-model parameter block (learned plan) or null
+// model: host copy of a cost-model parameter block (learned plan) or null.
+// hubs: false keeps every suffix whole in the middle-vertex walk (the plan the
+// cost model's features and cycle logs are taken on).
 int build_k3_plan(gary_graph *g, const PlanParams &pp, cudaStream_t s, gary_count_plan **out,
-                  const float *model = nullptr);
+                  const float *model = nullptr, bool hubs = true);
 // Cost-model features and legal-variant masks of every middle vertex.
 int k3_features(gary_graph *g, gary_count_plan *plan, float *d_x, uint8_t *d_legal, cudaStream_t s);
 int launch_k3(gary_graph *g, gary_count_plan *plan, unsigned long long *d_out, cudaStream_t s,
