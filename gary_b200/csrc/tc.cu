@@ -170,7 +170,9 @@ __global__ void k_classify(const uint2 *__restrict__ row, const uint32_t *__rest
       const bool warp_fits = bitmap || dv <= pp.warp_cap;
       const uint64_t build = bitmap ? (span >> 5) + dv : 4ull * dv;
       const bool pred = pcost && warp_fits;
-      const uint64_t cp = work[v] + build + pp.vertex_overhead;  // probe cost
+      // probe cost; a tiny vertex has no set, and each record costs it at
+      // least an octet
+      const uint64_t cp = dv <= kTinyOut ? work[v] + 8 * nin + 16 : work[v] + build + pp.vertex_overhead;
       // learned: predicted cycles, but never below the probe cost scaled to
       // the same tile target, so that no tile outgrows a plain one (a vertex
       // the model under-rates would otherwise end the launch alone)
@@ -389,7 +391,7 @@ int build_in_index(gary_graph *g, cudaStream_t s, const DevBuf<uint32_t> &len, I
 
 }  // namespace
 
-PlanParams resolve_params(PlanParams pp, uint64_t total_work) {
+PlanParams resolve_params(PlanParams pp, uint64_t total_work, uint64_t records) {
   // Measured on RMAT 18-24: the best warp tile holds about 1/32 of a resident
   // warp's share of the work (2^11 probes at RMAT-18 up to 2^15 at RMAT-22 and
   // above; larger tiles leave warps idle at the end, smaller ones pay the
@@ -401,6 +403,10 @@ PlanParams resolve_params(PlanParams pp, uint64_t total_work) {
     const uint64_t want = total_work / (slots * 32);
     uint64_t t = 1ull << 11;
     while (t < want && t < (1ull << 15)) t <<= 1;
+    // a graph too small to give every resident warp such a tile is cut into one
+    // tile per warp: its time is that of the longest chain of dependent loads
+    const uint64_t share = (total_work + 8 * records) / slots;
+    if (share < t) t = std::max<uint64_t>(share, 128);
     pp.warp_tile_cost = t;
   }
   return pp;
@@ -420,7 +426,7 @@ int build_k3_plan(gary_graph *g, const PlanParams &pp_in, cudaStream_t s, gary_c
     GARY_TRY(build_in_index(g, s, len, plan->in));
   }
   tr.mark("in-edge index");
-  const PlanParams pp = resolve_params(pp_in, plan->in.total_work);
+  const PlanParams pp = resolve_params(pp_in, plan->in.total_work, plan->in.records);
   plan->params = pp;
   GARY_TRY(plan->vclass.alloc_persistent(n));
   DevBuf<uint64_t> costV;  // cost of each light vertex, 0 for the others
@@ -782,6 +788,85 @@ __device__ __forceinline__ uint32_t warp_vertex(const GraphView &g, const uint2 
   return c;
 }
 
+// How many of the 8 ids a, b equal one of the 8 ids p, q.
+__device__ __forceinline__ uint32_t match_octets(const uint4 &a, const uint4 &b, const uint4 &p, const uint4 &q) {
+  auto in = [&](uint32_t x) -> uint32_t {
+    return x == p.x || x == p.y || x == p.z || x == p.w || x == q.x || x == q.y || x == q.z || x == q.w;
+  };
+  return in(a.x) + in(a.y) + in(a.z) + in(a.w) + in(b.x) + in(b.y) + in(b.z) + in(b.w);
+}
+
+// All in-edges of the tiny vertices among 32 light ones (lane's v, where
+// `tiny`), without a set: the 32 vertices' records are walked flattened, and
+// within a batch of 32 records their octets are, so every lane compares one
+// octet of a suffix with the one or two octets of N+(v).  Building a set costs
+// a vertex some thousands of cycles of dependent loads and shared-memory
+// passes whatever its size, which for these vertices is most of their time.
+// All 32 lanes must call.
+__device__ __forceinline__ uint32_t tiny_vertices(const GraphView &g, const uint2 *__restrict__ inedge,
+                                                  const uint64_t *__restrict__ inptr, uint32_t v, uint2 rv,
+                                                  bool tiny, int lane) {
+  // N+(v)'s padding equals a suffix's padding: the suffix's is lowered by one
+  // (still no vertex id), which is also what lanes without an octet hold.
+  constexpr uint32_t kNever = kSentinel - 1u;
+  const uint4 *adj4 = reinterpret_cast<const uint4 *>(g.adj);
+  const uint64_t ib = tiny ? inptr[v] : 0;
+  const uint32_t nin = tiny ? (uint32_t)(inptr[v + 1] - ib) : 0u;
+  const uint32_t incl = warp_inclusive_sum(nin, lane);
+  const uint32_t records = __shfl_sync(kFull, incl, 31);
+  // record of flattened position p: rbias + p (mod 2^32, as the octets below) of the owner
+  const uint32_t rbias = (uint32_t)ib - (incl - nin);
+  const uint32_t myset = (rv.x >> 1) | (rv.y > 8 ? 1u << 31 : 0u);  // N+(v)'s first octet; bit 31: it has two
+  WarpRuns runs(incl - nin, nin, lane);
+  uint32_t cnt = 0;
+  auto fetch = [&](uint32_t rb, uint2 &r, uint32_t &set) {
+    const int o = (int)runs.owner(rb);
+    const uint32_t k = __shfl_sync(kFull, rbias, o) + rb + lane;
+    set = __shfl_sync(kFull, myset, o);
+    r = rb + lane < records ? inedge[k] : make_uint2(0, 0);
+  };
+  uint2 r;
+  uint32_t set;
+  fetch(0, r, set);
+  for (uint32_t rb = 0; rb < records; rb += 32) {
+    uint2 rn = make_uint2(0, 0);
+    uint32_t setn = 0;
+    if (rb + 32 < records) fetch(rb + 32, rn, setn);
+    const uint32_t o0 = r.x >> 3;
+    const uint32_t no = r.y ? ((r.x + r.y + 7) >> 3) - o0 : 0u;
+    const uint32_t oincl = warp_inclusive_sum(no, lane);
+    const uint32_t total = __shfl_sync(kFull, oincl, 31);
+    const uint32_t bias = o0 - (oincl - no);
+    WarpOwners owners(oincl - no, lane);
+    for (uint32_t pb = 0; pb < total; pb += 32) {
+      const int o = (int)owners.owner(pb);
+      const uint32_t oc = __shfl_sync(kFull, bias, o) + pb + lane;
+      const uint32_t sx = __shfl_sync(kFull, set, o);
+      const bool on = pb + lane < total;
+      const uint4 never = make_uint4(kNever, kNever, kNever, kNever);
+      uint4 a = never, b = never, p = never, q = never;
+      const uint32_t so = sx & 0x7FFFFFFFu;
+      if (on) {
+        a = adj4[2 * (uint64_t)oc];
+        b = adj4[2 * (uint64_t)oc + 1];
+        p = adj4[2 * (uint64_t)so];
+        q = adj4[2 * (uint64_t)so + 1];
+        a.x = min(a.x, kNever); a.y = min(a.y, kNever); a.z = min(a.z, kNever); a.w = min(a.w, kNever);
+        b.x = min(b.x, kNever); b.y = min(b.y, kNever); b.z = min(b.z, kNever); b.w = min(b.w, kNever);
+        cnt += match_octets(a, b, p, q);
+        if (sx >> 31) {
+          p = adj4[2 * (uint64_t)so + 2];
+          q = adj4[2 * (uint64_t)so + 3];
+          cnt += match_octets(a, b, p, q);
+        }
+      }
+    }
+    r = rn;
+    set = setn;
+  }
+  return cnt;
+}
+
 template <int WARPS, int MINB>
 __global__ void __launch_bounds__(WARPS * 32, MINB)
     k_tc_mid(GraphView g, const uint2 *__restrict__ inedge, const uint64_t *__restrict__ inptr,
@@ -849,8 +934,35 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
       for (uint32_t ib = tl.v0; ib < tl.v1; ib += 32) {
         const uint32_t nb = min(32u, tl.v1 - ib);
         const uint32_t myv = lane < nb ? light[ib + lane] : 0u;
-        for (uint32_t k = 0; k < nb; ++k)
+        unsigned left = nb < 32 ? (1u << nb) - 1u : kFull;
+        // the tiny ones together, unless per-vertex results are asked for
+        bool together = !ctl.cycles;
+        uint32_t gid = 0;
+        if (together && ctl.gcount) {
+          gid = lane < nb ? ctl.gid[myv] : 0u;
+          const uint32_t g0 = __shfl_sync(kFull, gid, 0);
+          together = __all_sync(kFull, lane >= nb || gid == g0);
+          gid = g0;
+        }
+        if (together) {
+          const uint2 rv = lane < nb ? g.row[myv] : make_uint2(0, 0);
+          const bool tiny = rv.y - 1u < kTinyOut;
+          const unsigned tm = __ballot_sync(kFull, tiny);
+          if (tm) {
+            const uint32_t c = tiny_vertices(g, inedge, inptr, myv, rv, tiny, lane);
+            cnt += c;
+            if (ctl.gcount) {
+              const unsigned long long sum = warp_sum_u64(c);
+              if (lane == 0 && sum) atomicAdd(&ctl.gcount[gid], sum);
+            }
+            left &= ~tm;
+          }
+        }
+        while (left) {
+          const int k = __ffs(left) - 1;
+          left &= left - 1;
           cnt += warp_vertex(g, inedge, inptr, __shfl_sync(kFull, myv, k), 0, 0xFFFFFFFFu, tab, lane, ctl);
+        }
       }
     }
   }

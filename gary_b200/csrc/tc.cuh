@@ -15,6 +15,9 @@ namespace gary {
 constexpr int tc_warps(int min_blocks) { return min_blocks >= 3 ? 12 : 16; }
 constexpr int kTcMaxWarps = 16;
 constexpr uint32_t kWarpTableSlots = 1024;  // per-warp shared set (4 KB)
+// A light vertex with at most this many higher neighbours (two octets) is
+// counted without a set.
+constexpr uint32_t kTinyOut = 16;
 constexpr uint32_t kGroupTile = 0xFFFFFFFFu;
 constexpr uint32_t kMaxCountCtas = 1024;  // CTAs of a counting launch (SMs x resident CTAs)
 
@@ -63,9 +66,9 @@ struct PlanParams {
   uint32_t stage_polls = kSpinLimit;        // polls of the first staging wait
 };
 
-// The parameters a plan over `total_work` probes uses: explicit values as
-// given, the zeros resolved.
-PlanParams resolve_params(PlanParams pp, uint64_t total_work);
+// The parameters a plan over `total_work` probes in `records` suffixes uses:
+// explicit values as given, the zeros resolved.
+PlanParams resolve_params(PlanParams pp, uint64_t total_work, uint64_t records);
 
 // Process-wide tuning overrides (0 = keep the default), set by gary_tune().
 PlanParams tuned_params();
