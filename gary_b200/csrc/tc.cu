@@ -184,7 +184,8 @@ __global__ void k_classify(const uint2 *__restrict__ row, const uint32_t *__rest
         kc = (uint32_t)min_u64((c + pp.cta_tile_cost - 1) / pp.cta_tile_cost, nin);
       } else if (c > tw) {
         cls = kClassSplit;
-        kw = (uint32_t)min_u64((c + tw - 1) / tw, nin);
+        const uint64_t piece = max(tw, pp.split_floor * dv);  // every piece builds the set again
+        kw = (uint32_t)min_u64((c + piece - 1) / piece, nin);
       } else {
         cls = kClassLight;
         cl = c;
@@ -393,17 +394,25 @@ int build_in_index(gary_graph *g, cudaStream_t s, const DevBuf<uint32_t> &len, I
 }  // namespace
 
 PlanParams resolve_params(PlanParams pp, uint64_t total_work, uint64_t records) {
-  // Measured on RMAT 18-24: the best warp tile holds about 1/32 of a resident
-  // warp's share of the work (2^11 probes at RMAT-18 up to 2^15 at RMAT-22 and
-  // above; larger tiles leave warps idle at the end, smaller ones pay the
-  // per-tile cost), and three resident CTAs per SM (12 warps each, against two
-  // of 16) pay from about 2^31 probes (RMAT-22) on.
-  if (pp.min_blocks != 2 && pp.min_blocks != 3) pp.min_blocks = total_work >= (1ull << 31) ? 3 : 2;
+  // Three resident CTAs per SM of 12 warps beat two of 16 from some 2^26 probes
+  // on (ms a count, 3 / 2: RMAT-18 0.119 / 0.123, RMAT-20 0.514 / 0.537, RMAT-22
+  // 3.02 / 3.22, RMAT-24 ef32 65.5 / 72.4; RMAT-16 0.039 either way).
+  if (pp.min_blocks != 2 && pp.min_blocks != 3) pp.min_blocks = total_work >= (1ull << 26) ? 3 : 2;
+  const uint64_t slots = (uint64_t)sm_count() * tc_warps(pp.min_blocks) * pp.min_blocks;
+  // A vertex is split over tiles no finer than split_floor probes per id of its
+  // set, or building the set anew for every piece costs too much (RMAT-22 3.71
+  // ms with pieces of any size, 3.23 at 32 probes an id, 3.02 at 128); graphs
+  // with little work for each warp need the parallelism more (RMAT-16 0.0384
+  // ms at 16 and below, 0.0435 at 64).
+  pp.split_floor = total_work / slots >= (1ull << 12) ? 128 : 16;
   if (!pp.warp_tile_cost) {
-    const uint64_t slots = (uint64_t)sm_count() * tc_warps(pp.min_blocks) * pp.min_blocks;
-    const uint64_t want = total_work / (slots * 32);
+    // The best warp tile holds about 1/128 of a resident warp's share of the
+    // work, between 2^11 and 2^14 probes: larger tiles leave warps idle at the
+    // end (RMAT-23 9.16 ms at 1/32 up to 2^15, 8.0 at 1/128), smaller ones pay
+    // the per-tile cost.
+    const uint64_t want = total_work / (slots * 128);
     uint64_t t = 1ull << 11;
-    while (t < want && t < (1ull << 15)) t <<= 1;
+    while (t < want && t < (1ull << 14)) t <<= 1;
     // a graph too small to give every resident warp such a tile is cut into one
     // tile per warp: its time is that of the longest chain of dependent loads
     const uint64_t share = (total_work + 8 * records) / slots;

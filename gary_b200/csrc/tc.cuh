@@ -48,8 +48,8 @@ struct Tile {
 };
 
 // warp_tile_cost and min_blocks left at 0 follow the graph's total work
-// (resolve_params): about 32 warp tiles per resident warp, and 3 resident CTAs
-// per SM once there are 2^31 probes or more.
+// (resolve_params): about 128 warp tiles per resident warp, and 3 resident CTAs
+// per SM once there are 2^26 probes or more.
 //
 // cta_set_words and stage_polls change no plan, only how CTA tiles run; they
 // exist so that tests can reach every CTA set path on small graphs:
@@ -62,6 +62,7 @@ struct PlanParams {
   uint64_t warp_tile_cost = 0;              // target probes per warp tile (0: from the work)
   uint64_t cta_tile_cost = 1u << 20;        // target probes per CTA tile
   uint64_t vertex_overhead = 64;            // fixed cost of a middle vertex
+  uint64_t split_floor = 0;                 // least probes per id of N+(v) in a piece of a split vertex (from the work)
   uint32_t min_blocks = 0;                  // resident CTAs per SM, 2 or 3 (0: from the work)
   uint32_t cta_set_words = 0;               // 0: the CTA's whole shared buffer
   uint32_t stage_polls = kSpinLimit;        // polls of the first staging wait
