@@ -12,12 +12,24 @@
 //                         excluded ids -- the intersect_num family the
 //                         reference leaves commented out (Intersection.cuh:361-485)
 //
-// Pair work is handed to warps by a persistent queue (32 pairs per grab).
-// Variants:
-//   MERGE   warp merge path: 32-wide windows of A and B, each lane locates its
-//           A value in the B window with 5 shuffles, windows advance by ballots
+// CTAs claim chunks of pairs from a persistent queue and sort each chunk's
+// pairs by what they need:
+//   few ids (the shorter list at most kTinyKeys)  all such pairs of a warp
+//           flattened over its lanes, one key a lane, a binary search each
+//   long (more than kLongCost of work)  the whole CTA: every warp takes a part
+//           of the shorter list and the stretch of the longer list its values
+//           span
+//   the rest  one warp a pair
+// One warp per pair, whatever its size, left the last pairs of 65536 ids
+// running alone for 1.4 ms of a launch, and a warp with nothing but a few
+// dependent loads to do for most others (Zipf lengths: half the lists hold at
+// most 8 ids).  AUTO, ms before and now: 2^20 pairs counted 3.48 / 2.67 (85 %
+// of copy bandwidth in the lists' bytes), 50,001 pairs with lists 1.44 / 0.46.
+// Variants, for a pair or a part of one:
+//   MERGE   1024-id tiles of the longer list in shared memory, the shorter
+//           list's values searched in them 32 at a time
 //   SEARCH  lanes take the shorter list's values as keys and search the
-//           longer list: phase 1 in 256 shared samples, phase 2 in HBM
+//           longer list: phase 1 in shared samples, phase 2 in HBM
 //   BITMAP  the longer list as a shared-memory bitmap over 32K-value windows,
 //           the shorter list probed window by window
 //   AUTO    SEARCH when the longer list is much longer, else MERGE
@@ -33,10 +45,18 @@
 namespace gary {
 namespace {
 
-constexpr int kSoWarps = 8;
 constexpr uint32_t kSoWarpWords = 1024;  // per-warp shared words
 constexpr uint32_t kSearchSamples = 256;
 constexpr uint32_t kInf = 0xFFFFFFFFu;
+constexpr uint32_t kTinyKeys = 16;
+constexpr uint32_t kLongCost = 3072;  // ids read, or 8 per searched key
+// Pairs a CTA of `warps` warps claims at a time, at most.
+constexpr uint32_t chunk_pairs(int warps) { return warps <= 8 ? 128 : 224; }
+// Batches of fewer pairs run 16-warp CTAs: the long pairs end sooner, and there
+// are not enough pairs to hide them (ms, 16 / 8 warps: 50,001 Zipf pairs with
+// lists 0.45 / 0.61, 1,000 pairs 0.046 / 0.059, 200,000 pairs 0.45 / 0.50,
+// 300,000 pairs of up to 4096 ids 0.31 / 0.28, 2^20 pairs 2.72 / 2.60).
+constexpr uint64_t kManyPairs = 1ull << 18;
 
 struct PairView {
   const uint64_t *a_off, *b_off;
@@ -72,31 +92,63 @@ struct PairOut {
 
 __device__ __forceinline__ unsigned lanemask_lt(int lane) { return (1u << lane) - 1u; }
 
+// first index in [0, len) with l[i] >= x, by all 32 lanes together: each step
+// reads 32 evenly spaced ids (len 65536: 4 dependent loads instead of 16)
+__device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t *l, uint32_t len, uint32_t x, int lane) {
+  uint32_t b = 0, e = len;  // the answer is in [b, e]
+  while (e - b > 32) {
+    const uint32_t step = (e - b + 31) / 32;
+    const uint32_t at = min(b + (lane + 1) * step, e) - 1;  // last id of the lane's stretch
+    const unsigned below = __ballot_sync(kFull, l[at] < x);
+    const uint32_t k = __popc(below);  // stretches wholly below x
+    b = min(b + k * step, e);
+    e = min(b + step, e);
+  }
+  const bool below = b + lane < e && l[b + lane] < x;
+  return b + __popc(__ballot_sync(kFull, below));
+}
+
 // ---- MERGE ------------------------------------------------------------------
-__device__ uint32_t pair_merge(const uint32_t *A, uint32_t la, const uint32_t *B, uint32_t lb,
+__device__ uint32_t pair_merge(const uint32_t *S, uint32_t ls, const uint32_t *L, uint32_t ll, uint32_t *tile,
                                uint32_t *out, int lane) {
-  uint32_t i = 0, j = 0, found_total = 0;
-  while (i < la && j < lb) {
-    const uint32_t av = i + lane < la ? A[i + lane] : kInf;
-    const uint32_t bv = j + lane < lb ? B[j + lane] : kInf;
-    const uint32_t a_last = __shfl_sync(kFull, av, min(31u, la - i - 1));
-    const uint32_t b_last = __shfl_sync(kFull, bv, min(31u, lb - j - 1));
-    // position of av in the B window: last k with B[k] <= av
-    int lo = 0;
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1) {
-      const uint32_t v = __shfl_sync(kFull, bv, lo + step - 1);
-      if (v <= av) lo += step;
+  uint32_t si = 0, found_total = 0;
+  auto key = [&](uint32_t i) { return i < ls ? S[i] : 0u; };
+  uint32_t x = key(lane), xn = key(32 + lane);  // this window of S and the next, in flight
+  for (uint32_t li = 0; li < ll && si < ls; li += kSoWarpWords) {
+    const uint32_t n = min(kSoWarpWords, ll - li);
+    if (n == kSoWarpWords) {
+#pragma unroll 8
+      for (uint32_t k = 0; k < kSoWarpWords; k += 32) tile[k + lane] = L[li + k + lane];
+    } else {
+      for (uint32_t k = lane; k < n; k += 32) tile[k] = L[li + k];
     }
-    const uint32_t cand = __shfl_sync(kFull, bv, lo);
-    const uint32_t bprev = __shfl_sync(kFull, bv, lo > 0 ? lo - 1 : 0);
-    const bool done_a = av != kInf && av <= b_last;
-    const bool hit = done_a && (cand == av || (lo > 0 && bprev == av));
-    const unsigned hm = __ballot_sync(kFull, hit);
-    if (out && hit) out[found_total + __popc(hm & lanemask_lt(lane))] = av;
-    found_total += __popc(hm);
-    i += __popc(__ballot_sync(kFull, done_a));
-    j += __popc(__ballot_sync(kFull, bv != kInf && bv <= a_last));
+    __syncwarp();
+    const uint32_t last = tile[n - 1];
+    while (true) {
+      // S[si .. si + 32), in x; the values past this tile wait for the next
+      const bool in = si + lane < ls && x <= last;
+      uint32_t pos = 0;  // ids of the tile below x
+#pragma unroll
+      for (uint32_t step = kSoWarpWords / 2; step; step >>= 1) {
+        const uint32_t at = pos + step - 1;
+        if (at < n && tile[at] < x) pos += step;
+      }
+      const bool hit = in && pos < n && tile[pos] == x;
+      const unsigned hm = __ballot_sync(kFull, hit);
+      if (out && hit) out[found_total + __popc(hm & lanemask_lt(lane))] = x;
+      found_total += __popc(hm);
+      const uint32_t done = __popc(__ballot_sync(kFull, in));
+      si += done;
+      if (done == 32) {
+        x = xn;
+        xn = key(si + 32 + lane);
+      } else if (done) {
+        x = key(si + lane);
+        xn = key(si + 32 + lane);
+      }
+      if (done < 32 || si >= ls) break;
+    }
+    __syncwarp();
   }
   return found_total;
 }
@@ -104,13 +156,17 @@ __device__ uint32_t pair_merge(const uint32_t *A, uint32_t la, const uint32_t *B
 // ---- SEARCH (two-phase) ---------------------------------------------------
 __device__ uint32_t pair_search(const uint32_t *S, uint32_t ls, const uint32_t *L, uint32_t ll,
                                 uint32_t *cache, uint32_t *out, int lane) {
-  const uint32_t ns = ll < kSearchSamples ? ll : kSearchSamples;
+  // a few samples per key; each is a sector of HBM of its own
+  const uint32_t want = ls <= 32 ? 64u : ls <= 64 ? 128u : kSearchSamples;
+  const uint32_t ns = ll < want ? ll : want;
   for (uint32_t k = lane; k < ns; k += 32) cache[k] = L[(uint64_t)k * ll / ns];
   __syncwarp();
   uint32_t found_total = 0;
+  uint32_t xn = lane < ls ? S[lane] : 0u;
   for (uint32_t b = 0; b < ls; b += 32) {
     const bool ok = b + lane < ls;
-    const uint32_t x = ok ? S[b + lane] : 0u;
+    const uint32_t x = xn;
+    xn = b + 32 + lane < ls ? S[b + 32 + lane] : 0u;
     const bool hit = ok && search_2phase(L, ll, cache, ns, x);
     const unsigned hm = __ballot_sync(kFull, hit);
     if (out && hit) out[found_total + __popc(hm & lanemask_lt(lane))] = x;
@@ -167,74 +223,210 @@ __device__ uint32_t pair_bitmap(const uint32_t *S, uint32_t ls, const uint32_t *
   return found_total;
 }
 
+// A pair as the kernel runs it: S the shorter list (ties: A), L the longer.
+struct PairJob {
+  const uint32_t *S, *L;
+  uint32_t ls, ll;
+};
+
+__device__ __forceinline__ uint32_t warp_pair(int variant, const PairJob &j, uint32_t *mine, uint32_t *out, int lane) {
+  if (variant == GARY_ISECT_MERGE) return pair_merge(j.S, j.ls, j.L, j.ll, mine, out, lane);
+  if (variant == GARY_ISECT_SEARCH) return pair_search(j.S, j.ls, j.L, j.ll, mine, out, lane);
+  return pair_bitmap(j.S, j.ls, j.L, j.ll, mine, out, lane);
+}
+
+// AUTO searches once the longer list exceeds half of |S| log2 |L|.
+__device__ __forceinline__ int pair_variant(int variant, uint32_t ls, uint32_t ll) {
+  if (variant != GARY_ISECT_AUTO) return variant;
+  const uint32_t lg = 32 - __clz(ll);
+  return 2ull * ll > (uint64_t)ls * lg ? GARY_ISECT_SEARCH : GARY_ISECT_MERGE;
+}
+
+template <int kSoWarps>
 __global__ void __launch_bounds__(kSoWarps * 32)
-    k_intersect_pairs(PairView pv, uint64_t npairs, int variant, PairOut po, PairFilter pf,
+    k_intersect_pairs(PairView pv, uint64_t npairs, uint32_t chunk, int variant, PairOut po, PairFilter pf,
                       unsigned long long *queue, unsigned long long *total) {
-  __shared__ __align__(16) uint32_t smem[kSoWarps * kSoWarpWords];
+  extern __shared__ __align__(16) uint32_t smem[];  // kSoWarps * kSoWarpWords
+  constexpr uint32_t kChunkPairs = chunk_pairs(kSoWarps);
+  static_assert(kChunkPairs <= 256 && kChunkPairs <= kSoWarps * 32, "a thread per pair, numbered in a byte");
+  __shared__ PairJob jobs[kChunkPairs];
+  __shared__ uint32_t found[kChunkPairs];  // per pair of the chunk
+  __shared__ uint8_t mid[kChunkPairs], big[kChunkPairs];
+  __shared__ uint32_t n_mid, n_big, next_mid;
+  __shared__ uint32_t piece[kSoWarps];
+  __shared__ unsigned long long s_first;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t *mine = smem + warp * kSoWarpWords;
   for (uint32_t i = lane; i < kSoWarpWords; i += 32) mine[i] = 0u;
-  __syncwarp();
   unsigned long long local = 0;
-  // One pair per claim: with Zipf lengths, claims of 32 pairs left warps
-  // finishing their last long pairs while the rest idled (2^20 pairs at
-  // overlap 0.1: AUTO 174 M pairs/s with 32 per claim, 214 M with 2, 235 M
-  // with 1; one queue atomic per pair is far below what the L2 serves).
   while (true) {
-    unsigned long long c = 0;
-    if (lane == 0) c = atomicAdd(queue, 1ull);
-    c = __shfl_sync(kFull, c, 0);
-    if (c >= npairs) break;
-    {
-      const uint64_t p = c;
+    if (threadIdx.x == 0) {
+      s_first = atomicAdd(queue, (unsigned long long)chunk);
+      n_mid = n_big = next_mid = 0;
+    }
+    __syncthreads();
+    const uint64_t first = s_first;
+    if (first >= npairs) break;
+    const uint32_t np = (uint32_t)min((unsigned long long)chunk, (unsigned long long)(npairs - first));
+    if (threadIdx.x < np) {
+      const uint64_t p = first + threadIdx.x;
       uint32_t la = pv.a_len[p], lb = pv.b_len[p];
       const uint32_t *A = pv.a + pv.a_off[p], *B = pv.b + pv.b_off[p];
-      const uint32_t bound = pf.bound ? pf.bound[p] : kInf;
       if (pf.bound) {  // members < bound only: both lists end at the bound
+        const uint32_t bound = pf.bound[p];
         la = so_lower_bound(A, la, bound);
         lb = so_lower_bound(B, lb, bound);
       }
-      uint32_t *out = po.out_off ? po.out + po.out_off[p] : nullptr;
-      uint32_t c2 = 0;
-      if (la && lb) {
-        // S: shorter (ties: A), L: longer
-        const bool a_short = la <= lb;
-        const uint32_t *S = a_short ? A : B, *L = a_short ? B : A;
-        const uint32_t ls = a_short ? la : lb, ll = a_short ? lb : la;
-        int v = variant;
-        if (v == GARY_ISECT_AUTO) {
-          // search once the longer list exceeds half of |S| log2 |L| (measured
-          // on 2^20 Zipf pairs at overlap 0.1: 239 M pairs/s with the cut at
-          // 4 |S| log2 |L|, 285 M at 1x, 301 M at 1/2, 290 M at 1/4)
-          const uint32_t lg = 32 - __clz(ll);
-          v = 2ull * ll > (uint64_t)ls * lg ? GARY_ISECT_SEARCH : GARY_ISECT_MERGE;
-        }
-        if (v == GARY_ISECT_MERGE) c2 = pair_merge(S, ls, L, ll, out, lane);
-        else if (v == GARY_ISECT_SEARCH) c2 = pair_search(S, ls, L, ll, mine, out, lane);
-        else {
-          c2 = pair_bitmap(S, ls, L, ll, mine, out, lane);
-        }
+      const bool a_short = la <= lb;
+      const PairJob j{a_short ? A : B, a_short ? B : A, a_short ? la : lb, a_short ? lb : la};
+      jobs[threadIdx.x] = j;
+      found[threadIdx.x] = 0;
+      if (j.ls > kTinyKeys) {
+        // work in loads: a search's keys cost several each
+        const uint64_t cost = pair_variant(variant, j.ls, j.ll) == GARY_ISECT_SEARCH ? 8ull * j.ls : (uint64_t)j.ls + j.ll;
+        if (cost > kLongCost) big[atomicAdd(&n_big, 1u)] = (uint8_t)threadIdx.x;
+        else mid[atomicAdd(&n_mid, 1u)] = (uint8_t)threadIdx.x;
       }
-      if (pf.ex_off && la && lb) {  // excluded ids that are members (each id once)
-        const uint64_t e0 = pf.ex_off[p], e1 = pf.ex_off[p + 1];
+    }
+    __syncthreads();
+    {  // pairs of few ids: this warp's share of the chunk, one key a lane
+      const uint32_t share = (np + kSoWarps - 1) / kSoWarps, q0 = warp * share;
+      const uint32_t ls = lane < share && q0 + lane < np ? jobs[q0 + lane].ls : 0u;
+      const uint32_t keys = ls <= kTinyKeys ? ls : 0u;
+      const uint32_t incl = warp_inclusive_sum(keys, lane);
+      const uint32_t all = __shfl_sync(kFull, incl, 31);
+      WarpRuns runs(incl - keys, keys, lane);
+      for (uint32_t pb = 0; pb < all; pb += 32) {
+        const int o = (int)runs.owner(pb);
+        const uint32_t start = __shfl_sync(kFull, incl - keys, o);
+        const bool on = pb + lane < all;
+        bool hit = false;
+        uint32_t x = 0;
+        if (on) {
+          const PairJob j = jobs[q0 + o];
+          x = j.S[pb + lane - start];
+          uint32_t base = 0;
+          for (uint32_t n = j.ll; n > 1;) {  // ids below x: at least base, at most base + n - 1 but for the last
+            const uint32_t half = n >> 1;
+            if (j.L[base + half - 1] < x) base += half;
+            n -= half;
+          }
+          hit = j.L[base] == x;
+        }
+        const unsigned hm = __ballot_sync(kFull, hit);
+        // the lanes of this pair in the batch: from its first key on
+        const uint32_t from = start > pb ? start - pb : 0u;
+        const unsigned before = hm & lanemask_lt(lane) & ~lanemask_lt(from);
+        const uint32_t had = on ? found[q0 + o] : 0u;
+        if (po.out_off && hit) po.out[po.out_off[first + q0 + o] + had + __popc(before)] = x;
+        __syncwarp();
+        const int next = __shfl_down_sync(kFull, on ? o : -1, 1);
+        if (on && (lane == 31 || next != o)) found[q0 + o] = had + __popc(before) + hit;
+        __syncwarp();
+      }
+    }
+    while (true) {  // one warp a pair
+      uint32_t m = 0;
+      if (lane == 0) m = atomicAdd(&next_mid, 1u);
+      m = __shfl_sync(kFull, m, 0);
+      if (m >= n_mid) break;
+      const uint32_t q = mid[m];
+      const PairJob j = jobs[q];
+      uint32_t *out = po.out_off ? po.out + po.out_off[first + q] : nullptr;
+      const uint32_t c = warp_pair(pair_variant(variant, j.ls, j.ll), j, mine, out, lane);
+      if (lane == 0) found[q] = c;
+    }
+    for (uint32_t i = 0; i < n_big; ++i) {  // the CTA together, a part of S a warp
+      const uint32_t q = big[i];
+      const PairJob j = jobs[q];
+      const int v = pair_variant(variant, j.ls, j.ll);
+      const uint32_t s0 = (uint32_t)((uint64_t)j.ls * warp / kSoWarps), s1 = (uint32_t)((uint64_t)j.ls * (warp + 1) / kSoWarps);
+      PairJob sub{nullptr, nullptr, 0, 0};
+      if (s0 < s1) {  // more ids than warps: always
+        const uint32_t l0 = warp_lower_bound(j.L, j.ll, j.S[s0], lane);
+        const uint32_t l1 = l0 + warp_lower_bound(j.L + l0, j.ll - l0, j.S[s1 - 1], lane);
+        sub = PairJob{j.S + s0, j.L + l0, s1 - s0, min(l1 + 1, j.ll) - l0};
+      }
+      uint32_t c = 0;
+      if (sub.ll) c = warp_pair(v, sub, mine, nullptr, lane);
+      if (!po.out_off) {
+        if (lane == 0 && c) atomicAdd(&found[q], c);
+        continue;
+      }
+      // the places of the parts follow from their counts: a second pass writes
+      if (lane == 0) piece[warp] = c;
+      __syncthreads();
+      uint32_t at = 0, sum = 0;
+      for (int w = 0; w < kSoWarps; ++w) {
+        at += w < warp ? piece[w] : 0u;
+        sum += piece[w];
+      }
+      if (c) warp_pair(v, sub, mine, po.out + po.out_off[first + q] + at, lane);
+      if (threadIdx.x == 0) found[q] = sum;
+      __syncthreads();
+    }
+    __syncthreads();
+    if (pf.ex_off) {  // excluded ids that are members (each id once)
+      for (uint32_t q = warp; q < np; q += kSoWarps) {
+        const PairJob j = jobs[q];
+        if (!j.ls) continue;
+        const uint64_t e0 = pf.ex_off[first + q], e1 = pf.ex_off[first + q + 1];
+        const uint32_t bound = pf.bound ? pf.bound[first + q] : kInf;
         uint32_t drop = 0;
         for (uint64_t k = e0 + lane; k < e1; k += 32) {
           const uint32_t x = pf.ex[k];
-          bool first = x < bound;
-          for (uint64_t j = e0; first && j < k; ++j) first = pf.ex[j] != x;
-          if (first) {
-            const uint32_t ia = so_lower_bound(A, la, x), ib = so_lower_bound(B, lb, x);
-            drop += ia < la && A[ia] == x && ib < lb && B[ib] == x;
+          bool is_first = x < bound;
+          for (uint64_t i = e0; is_first && i < k; ++i) is_first = pf.ex[i] != x;
+          if (is_first) {
+            const uint32_t is = so_lower_bound(j.S, j.ls, x), il = so_lower_bound(j.L, j.ll, x);
+            drop += is < j.ls && j.S[is] == x && il < j.ll && j.L[il] == x;
           }
         }
         for (int o = 16; o; o >>= 1) drop += __shfl_xor_sync(kFull, drop, o);
-        c2 -= drop;
+        if (lane == 0) found[q] -= drop;
       }
-      if (lane == 0 && po.counts) po.counts[p] = c2;
-      local += c2;
+      __syncthreads();
     }
+    if (threadIdx.x < np) {
+      const uint32_t c = found[threadIdx.x];
+      if (po.counts) po.counts[first + threadIdx.x] = c;
+      local += c;
+    }
+    // the next chunk's set-up is ordered after these reads by its claim's barrier
   }
+  local = warp_sum_u64(local);
   if (lane == 0 && total && local) atomicAdd(total, local);
+}
+
+// One launch over all pairs.
+template <int W>
+int launch_pairs(const PairView &pv, uint64_t npairs, int variant, const PairOut &po, const PairFilter &pf,
+                 uint64_t *d_queue, uint64_t *d_total, cudaStream_t s) {
+  constexpr size_t smem = (size_t)W * kSoWarpWords * 4;
+  auto kern = k_intersect_pairs<W>;
+  static bool done[64] = {false};  // shared memory beyond the default limit, once per device
+  const int dev = device_ordinal();
+  if (dev >= 64 || !done[dev]) {
+    GARY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (dev < 64) done[dev] = true;
+  }
+  int per_sm = 0;
+  GARY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, W * 32, smem));
+  if (per_sm < 1) per_sm = 1;
+  const unsigned grid = (unsigned)(sm_count() * per_sm);
+  // pairs per claim: some claims for every CTA, a pair for every warp
+  const uint64_t c = npairs / ((W > 8 ? 2ull : 4ull) * grid);
+  const uint32_t chunk = c < W ? (uint32_t)W : c > chunk_pairs(W) ? chunk_pairs(W) : (uint32_t)c;
+  kern<<<grid, W * 32, smem, s>>>(pv, npairs, chunk, variant, po, pf, reinterpret_cast<unsigned long long *>(d_queue),
+                                  reinterpret_cast<unsigned long long *>(d_total));
+  GARY_CUDA(cudaGetLastError());
+  return GARY_OK;
+}
+
+int launch_pairs_any(const PairView &pv, uint64_t npairs, int variant, const PairOut &po, const PairFilter &pf,
+                     uint64_t *d_queue, uint64_t *d_total, cudaStream_t s) {
+  return npairs >= kManyPairs ? launch_pairs<8>(pv, npairs, variant, po, pf, d_queue, d_total, s)
+                              : launch_pairs<16>(pv, npairs, variant, po, pf, d_queue, d_total, s);
 }
 
 // ---- search batch ----------------------------------------------------------
@@ -399,16 +591,9 @@ extern "C" int gary_intersect_batch(uint64_t npairs, const uint64_t *d_a_off, co
   GARY_CUDA(cudaMemsetAsync(d_queue, 0, 8, s));
   if (d_total) GARY_CUDA(cudaMemsetAsync(d_total, 0, 8, s));
   if (!npairs) return GARY_OK;
-  int per_sm = 0;
-  GARY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_intersect_pairs, kSoWarps * 32, 0));
-  if (per_sm < 1) per_sm = 1;
   const PairView pv{d_a_off, d_b_off, d_a_len, d_b_len, d_a, d_b};
   const PairOut po{d_counts, d_out_off, d_out};
-  k_intersect_pairs<<<(unsigned)(sm_count() * per_sm), kSoWarps * 32, 0, s>>>(
-      pv, npairs, variant, po, PairFilter{nullptr, nullptr, nullptr},
-      reinterpret_cast<unsigned long long *>(d_queue), reinterpret_cast<unsigned long long *>(d_total));
-  GARY_CUDA(cudaGetLastError());
-  return GARY_OK;
+  return launch_pairs_any(pv, npairs, variant, po, PairFilter{nullptr, nullptr, nullptr}, d_queue, d_total, s);
 }
 
 extern "C" int gary_intersect_num_batch(uint64_t npairs, const uint64_t *d_a_off, const uint32_t *d_a_len,
@@ -427,16 +612,9 @@ extern "C" int gary_intersect_num_batch(uint64_t npairs, const uint64_t *d_a_off
   GARY_CUDA(cudaMemsetAsync(d_queue, 0, 8, s));
   if (d_total) GARY_CUDA(cudaMemsetAsync(d_total, 0, 8, s));
   if (!npairs) return GARY_OK;
-  int per_sm = 0;
-  GARY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_intersect_pairs, kSoWarps * 32, 0));
-  if (per_sm < 1) per_sm = 1;
   const PairView pv{d_a_off, d_b_off, d_a_len, d_b_len, d_a, d_b};
   const PairOut po{d_counts, nullptr, nullptr};
-  k_intersect_pairs<<<(unsigned)(sm_count() * per_sm), kSoWarps * 32, 0, s>>>(
-      pv, npairs, variant, po, PairFilter{d_bound, d_ex_off, d_ex},
-      reinterpret_cast<unsigned long long *>(d_queue), reinterpret_cast<unsigned long long *>(d_total));
-  GARY_CUDA(cudaGetLastError());
-  return GARY_OK;
+  return launch_pairs_any(pv, npairs, variant, po, PairFilter{d_bound, d_ex_off, d_ex}, d_queue, d_total, s);
 }
 
 extern "C" int gary_search_batch(const uint32_t *d_list, uint64_t len, const uint32_t *d_keys,

@@ -264,8 +264,8 @@ int gary_graph_drop_plans(gary_graph *g);
 /* ---- batched set operations: the include/ops layer ---------------------
  * Lists are sorted ascending, values < UINT32_MAX. */
 #define GARY_ISECT_AUTO 0   /* SEARCH when 2|L| > |S| log2 |L| (L the longer list), else MERGE */
-#define GARY_ISECT_MERGE 1  /* warp merge path over 32-wide windows (ballot / shuffle) */
-#define GARY_ISECT_SEARCH 2 /* two-phase search: 256 shared samples, then HBM */
+#define GARY_ISECT_MERGE 1  /* the shorter list searched in 1024-id shared tiles of the longer one */
+#define GARY_ISECT_SEARCH 2 /* two-phase search: up to 256 shared samples, then HBM */
 #define GARY_ISECT_BITMAP 3 /* shared bitmap of the longer list over 32K-value windows */
 
 /* |A_i & B_i| for npairs pairs; A_i = d_a[d_a_off[i] .. + d_a_len[i]), B_i likewise.
