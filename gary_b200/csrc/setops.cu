@@ -188,18 +188,12 @@ __device__ uint32_t pair_bitmap(const uint32_t *S, uint32_t ls, const uint32_t *
     const uint32_t s0 = S[si], l0 = L[li];
     const uint32_t w0 = (s0 > l0 ? s0 : l0) / W * W;  // window holding the larger head
     const uint64_t w1 = (uint64_t)w0 + W;
-    // skip values below the window
-    auto lower = [&](const uint32_t *X, uint32_t n, uint32_t from, uint64_t v) {
-      uint32_t b = from, e = n;  // first index with X[idx] >= v
-      while (b < e) {
-        const uint32_t mid = (b + e) >> 1;
-        if (X[mid] < v) b = mid + 1;
-        else e = mid;
-      }
-      return b;
+    // skip values below the window, and find its end
+    auto from = [&](const uint32_t *X, uint32_t n, uint32_t i, uint64_t v) {
+      return v > kInf ? n : i + warp_lower_bound(X + i, n - i, (uint32_t)v, lane);
     };
-    const uint32_t sb = lower(S, ls, si, w0), se = lower(S, ls, sb, w1);
-    const uint32_t lb = lower(L, ll, li, w0), le = lower(L, ll, lb, w1);
+    const uint32_t sb = from(S, ls, si, w0), se = from(S, ls, sb, w1);
+    const uint32_t lb = from(L, ll, li, w0), le = from(L, ll, lb, w1);
     for (uint32_t k = lb + lane; k < le; k += 32) {
       const uint32_t o = L[k] - w0;
       atomicOr(&bm[o >> 5], 1u << (o & 31));
@@ -282,8 +276,10 @@ __global__ void __launch_bounds__(kSoWarps * 32)
       jobs[threadIdx.x] = j;
       found[threadIdx.x] = 0;
       if (j.ls > kTinyKeys) {
-        // work in loads: a search's keys cost several each
-        const uint64_t cost = pair_variant(variant, j.ls, j.ll) == GARY_ISECT_SEARCH ? 8ull * j.ls : (uint64_t)j.ls + j.ll;
+        // work in loads: a search's keys cost several each, and a bitmap's may
+        // each lie in a window of its own
+        const int v = pair_variant(variant, j.ls, j.ll);
+        const uint64_t cost = v == GARY_ISECT_SEARCH ? 8ull * j.ls : v == GARY_ISECT_BITMAP ? 64ull * j.ls : (uint64_t)j.ls + j.ll;
         if (cost > kLongCost) big[atomicAdd(&n_big, 1u)] = (uint8_t)threadIdx.x;
         else mid[atomicAdd(&n_mid, 1u)] = (uint8_t)threadIdx.x;
       }
