@@ -185,7 +185,66 @@ void persistent_free(void *p) {
   if (cur != info.dev) cudaSetDevice(cur);
 }
 
+// ---- pinned result slots ---------------------------------------------------
+// Where gary_count reads a launch's scheduler words and count to: page-locked,
+// so that the copy is one asynchronous operation on the stream instead of a
+// staged copy the host waits in.  One page for the process, handed out slot by
+// slot under a lock, returned to the driver by release_cached_memory while no
+// slot is out.  With no slot free the caller's own (pageable) struct is used.
+struct ResultWords {
+  SchedState st;
+};
+
+namespace {
+constexpr int kResultSlots = 32;
+std::mutex g_slot_mu;
+ResultWords *g_slots = nullptr;
+uint32_t g_slots_used = 0;
+}  // namespace
+
+struct ResultSlot {
+  ResultWords own{};
+  ResultWords *p = &own;
+  int index = -1;
+  ResultSlot() {
+    std::lock_guard<std::mutex> lk(g_slot_mu);
+    if (!g_slots && cudaHostAlloc(reinterpret_cast<void **>(&g_slots), sizeof(ResultWords) * kResultSlots,
+                                  cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      g_slots = nullptr;
+      return;
+    }
+    for (int k = 0; k < kResultSlots; ++k)
+      if (!((g_slots_used >> k) & 1u)) {
+        g_slots_used |= 1u << k;
+        index = k;
+        p = g_slots + k;
+        return;
+      }
+  }
+  ResultSlot(const ResultSlot &) = delete;
+  ResultSlot &operator=(const ResultSlot &) = delete;
+  ResultWords *operator->() { return p; }
+  // Gives the slot back, once no copy into it can be in flight.  A call that
+  // fails before that keeps it out: at most kResultSlots such calls, and the
+  // ones after them use their own struct.
+  void done() {
+    if (index < 0) return;
+    std::lock_guard<std::mutex> lk(g_slot_mu);
+    g_slots_used &= ~(1u << index);
+    index = -1;
+    p = &own;
+  }
+};
+
 void release_cached_memory() {
+  {
+    std::lock_guard<std::mutex> lk(g_slot_mu);
+    if (g_slots && !g_slots_used) {
+      cudaFreeHost(g_slots);
+      g_slots = nullptr;
+    }
+  }
   {
     std::lock_guard<std::mutex> lk(g_blk_mu);
     for (int d = 0; d < 64; ++d) trim_blocks_locked(d, 0);
@@ -292,16 +351,22 @@ std::mutex g_tuning_mu;
 std::vector<float> g_model;  // process-wide cost model (gary_set_cost_model)
 std::mutex g_model_mu;
 
+// own_word: the caller has no device word; a triangle count goes to the
+// plan's SchedState::total (d_out is then the word of the other patterns).
 int count_async(gary_graph *g, int pattern, int sched, cudaStream_t s, unsigned long long *d_out,
-                uint32_t shard = 0, uint32_t nshards = 1) {
+                uint32_t shard = 0, uint32_t nshards = 1, bool own_word = false) {
   GARY_CHECK_ARG(g != nullptr, "graph is NULL");
-  GARY_CHECK_ARG(d_out != nullptr, "output pointer is NULL");
+  GARY_CHECK_ARG(d_out != nullptr || own_word, "output pointer is NULL");
   GARY_CHECK_ARG(pattern == GARY_PATTERN_TRIANGLE || pattern == GARY_PATTERN_4CYCLE ||
                      pattern == GARY_PATTERN_4CLIQUE,
                  "unknown pattern %d", pattern);
   GARY_CHECK_ARG(sched == GARY_SCHED_PLAIN || sched == GARY_SCHED_LEARNED, "unknown scheduler %d",
                  sched);
   GARY_CHECK_ARG(nshards >= 1 && shard < nshards, "shard %u of %u is out of range", shard, nshards);
+  if (own_word && pattern != GARY_PATTERN_TRIANGLE) {
+    if (!g->result.p) GARY_TRY(g->result.alloc_persistent(1));
+    d_out = g->result.p;
+  }
   if (pattern == GARY_PATTERN_4CLIQUE) {
     if (g->dag.max_len > kK4MaxOutDegree) {
       set_error("4-clique counting supports out-degree <= %u (graph has %u)", kK4MaxOutDegree,
@@ -596,14 +661,16 @@ extern "C" int gary_count(gary_graph *g, int pattern, int sched, void *stream, u
   GARY_CHECK_ARG(g != nullptr, "graph is NULL");
   return guarded("gary_count", [&] {
     cudaStream_t s = gary::as_stream(stream);
-    if (!g->result.p) GARY_TRY(g->result.alloc_persistent(1));
-    GARY_TRY(gary::count_async(g, pattern, sched, s, g->result.p));
-    unsigned long long h = 0;
-    gary::SchedState st{};
-    GARY_CUDA(cudaMemcpyAsync(&h, g->result.p, sizeof(h), cudaMemcpyDeviceToHost, s));
-    GARY_CUDA(cudaMemcpyAsync(&st, g->last_sched, sizeof(st), cudaMemcpyDeviceToHost, s));
+    GARY_TRY(gary::count_async(g, pattern, sched, s, nullptr, 0, 1, true));
+    gary::ResultSlot slot;
+    GARY_CUDA(cudaMemcpyAsync(&slot->st, g->last_sched, sizeof(gary::SchedState), cudaMemcpyDeviceToHost, s));
+    if (pattern != GARY_PATTERN_TRIANGLE)
+      GARY_CUDA(cudaMemcpyAsync(&slot->st.total, g->result.p, 8, cudaMemcpyDeviceToHost, s));
     GARY_CUDA(cudaStreamSynchronize(s));
+    const gary::SchedState st = slot->st;
+    slot.done();
     GARY_TRY(gary::launch_status(st.error));
+    const unsigned long long h = st.total;
     *out = h;
     return GARY_OK;
   });

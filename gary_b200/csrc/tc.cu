@@ -513,7 +513,8 @@ int build_k3_plan(gary_graph *g, const PlanParams &pp_in, cudaStream_t s, gary_c
     k_fill_group_tiles<<<grid_for(G), kThreads, 0, s>>>(starts.p, G, L, plan->tiles.p + nC + nW);
     GARY_CUDA(cudaGetLastError());
   }
-  GARY_TRY(plan->sched.alloc_persistent(1));
+  constexpr size_t kSpanBytes = 2ull * kMaxCountCtas * 8;
+  GARY_TRY(plan->sched.alloc_persistent(1 + (kSpanBytes + sizeof(SchedState) - 1) / sizeof(SchedState)));
   GARY_CUDA(cudaStreamSynchronize(s));
   tr.mark("tiles");
   *out = plan.release();
@@ -1010,18 +1011,18 @@ int launch_k3_impl(gary_graph *g, gary_count_plan *plan, unsigned long long *d_o
   constexpr int WARPS = tc_warps(MINB);
   auto kern = k_tc_mid<WARPS, MINB>;
   const size_t smem = (size_t)(WARPS + 1) * kWarpTableSlots * 4;  // + 1: regions start on a multiple of their size
-  static bool attr_done[64] = {false};
+  // the resident CTAs per SM, asked for once per device
+  static int resident[64] = {0};
   const int dev = device_ordinal();
-  if (dev < 64 && !attr_done[dev]) {
+  int per_sm = dev < 64 ? resident[dev] : 0;
+  if (!per_sm) {
     GARY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_done[dev] = true;
+    GARY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WARPS * 32, smem));
+    if (per_sm < 1) per_sm = 1;
+    if (dev < 64) resident[dev] = per_sm;
   }
-  int per_sm = 0;
-  GARY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WARPS * 32, smem));
-  if (per_sm < 1) per_sm = 1;
   const unsigned grid = (unsigned)std::min<int>(sm_count() * per_sm, (int)kMaxCountCtas);
-  if (!plan->span.p) GARY_TRY(plan->span.alloc_persistent(2 * kMaxCountCtas));
-  ctl.span = plan->span.p;
+  ctl.span = plan->span();
   const TileRange rng = shard_range(plan->n_cta, plan->n_warp, shard, nshards);
   auto part = [&](uint32_t k) { return (uint32_t)((uint64_t)plan->hub.n_list * k / nshards); };
   const HubView hub{plan->hub.rows.p, plan->hub.rowof.p, plan->hub.list.p, plan->hub.cut.p, plan->hub.first, part(shard), part(shard + 1)};
@@ -1031,9 +1032,9 @@ int launch_k3_impl(gary_graph *g, gary_count_plan *plan, unsigned long long *d_o
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   GARY_CUDA(cudaStreamIsCapturing(s, &cap));
   const bool timed = cap == cudaStreamCaptureStatusNone;
-  GARY_CUDA(cudaMemsetAsync(plan->sched.p, 0, sizeof(SchedState), s));
-  GARY_CUDA(cudaMemsetAsync(plan->span.p, 0, 2ull * grid * 8, s));
-  GARY_CUDA(cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), s));
+  GARY_CUDA(cudaMemsetAsync(plan->sched.p, 0, sizeof(SchedState) + 2ull * grid * 8, s));
+  if (d_out) GARY_CUDA(cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), s));
+  else d_out = &plan->sched.p->total;
   if (timed) GARY_CUDA(cudaEventRecord(g->ev0, s));
   kern<<<grid, WARPS * 32, smem, s>>>(g->view(), plan->in.inedge.p, plan->in.inptr.p, plan->light.p,
                                       plan->tiles.p, plan->n_cta, rng, hub, plan->sched.p, d_out, ctl, cfg);
@@ -1045,7 +1046,7 @@ int launch_k3_impl(gary_graph *g, gary_count_plan *plan, unsigned long long *d_o
   g->last.work = plan->in.total_work + plan->in.hub_work;
   g->last_timed = timed;
   g->last_sched = plan->sched.p;
-  g->last_span = plan->span.p;
+  g->last_span = plan->span();
   g->last_span_ctas = grid;
   return GARY_OK;
 }

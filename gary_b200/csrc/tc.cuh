@@ -92,6 +92,7 @@ inline TileRange shard_range(uint32_t n_cta, uint32_t n_warp, uint32_t shard, ui
 
 // Scheduler words, zeroed before every launch.
 struct SchedState {
+  unsigned long long total;  // the count, for a caller without a device word of its own
   uint32_t next_cta;
   uint32_t next_warp;
   uint32_t error;     // kLaunchErr* bits
@@ -129,11 +130,12 @@ struct gary_count_plan {
   gary::DevBuf<gary::Tile> tiles;
   uint32_t n_cta = 0;
   uint32_t n_warp = 0;
+  // scheduler words, then per CTA of the last launch its start and finish time
+  // (%globaltimer ns): one block, so that one memset clears both
   gary::DevBuf<gary::SchedState> sched;
+  unsigned long long *span() const { return reinterpret_cast<unsigned long long *>(sched.p + 1); }
   gary::DevBuf<uint8_t> variant;  // learned plans: intersection variant per middle vertex
   bool learned = false;
-  // per CTA of the last launch: start and finish time (%globaltimer ns)
-  gary::DevBuf<unsigned long long> span;
 };
 
 namespace gary {
@@ -144,6 +146,7 @@ int build_k3_plan(gary_graph *g, const PlanParams &pp, cudaStream_t s, gary_coun
                   const float *model = nullptr, bool hubs = true);
 // Cost-model features and legal-variant masks of every middle vertex.
 int k3_features(gary_graph *g, gary_count_plan *plan, float *d_x, uint8_t *d_legal, cudaStream_t s);
+// d_out null: the count goes to the plan's own SchedState::total.
 int launch_k3(gary_graph *g, gary_count_plan *plan, unsigned long long *d_out, cudaStream_t s,
               uint32_t shard, uint32_t nshards);
 // The same launch with a forced per-vertex variant array and/or a per-vertex
