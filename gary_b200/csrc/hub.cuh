@@ -56,6 +56,29 @@ struct HubView {
   uint32_t first, lo, hi;  // this launch counts list[lo .. hi)
 };
 
+// Adjacency rows for the 4-clique kernels: bit p of v's row says that v has the
+// higher neighbour first + p.  As HubRows, over a wider range of ids (memory
+// and the build grow with it, a look-up does not), without a counted list.
+struct AdjRows {
+  DevBuf<uint4> rows;
+  DevBuf<uint32_t> rowof;  // per vertex below `first`: its row, or kNoHubRow
+  DevBuf<uint32_t> low;    // per vertex: how many of its higher neighbours the rows do not cover
+  uint32_t first = 0;
+  uint32_t words = 0;      // per row; 0: no rows
+};
+
+// RMAT-22 ef16, ms per count of 4-cliques: 45.1 with rows of 8192 ids, 33.4 with
+// 16384, 31.0 with 32768 (twice the memory: 1.2 GB); 119.5 without rows.
+constexpr uint32_t kAdjRowIds = 16384;
+// Top neighbours a row needs (8 / 16 / 32 / 64: RMAT-22 ef16 33.1 / 33.2 / 33.4 /
+// 37.9 ms, RMAT-20 ef5 0.73 / 0.74 / 0.78 / 0.79).
+constexpr uint32_t kAdjMin = 16;
+
+// Builds them when at least an eighth of the pairs of higher neighbours have
+// their second id among the top ids and their first vertex a row; words stays 0
+// otherwise (sparse graphs without hubs: walking lists is cheaper there).
+int build_adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj);
+
 // Builds the rows of g's DAG when they pay, and len[u], the part of N+(u) the
 // middle-vertex walk still covers (all of it for a vertex not counted here).
 // Otherwise leaves hub.n_list 0 and len empty.

@@ -7,9 +7,13 @@
 // u < v < w < x is counted once at its lowest vertex u, as a triangle of the
 // subgraph induced by N+(u).  For every u (d = d+(u) ids) the kernel builds
 // that subgraph's upper-triangular adjacency as d bit rows of ceil(d/32)
-// words: row i has bit j set when N+(u)[j] is in N+(N+(u)[i]).  Rows are
-// filled by streaming each N+(v), v in N+(u), up to the largest id of N+(u)
-// and looking every id up in a shared id -> position hash of N+(u).  Then
+// words: row i has bit j set when N+(u)[j] is in N+(N+(u)[i]).  Columns whose
+// ids are among the graph's top 16384 are read off adjacency rows (hub.cuh), a
+// load and a ballot per 32 pairs; the others are filled by streaming each
+// N+(v), v in N+(u), up to the largest such id and looking every id up in a
+// shared id -> position hash.  (All columns by hash: 119.5 ms at RMAT-22 ef16;
+// top columns by rows 50.6 ms; and the lanes of a warp counting the same word of
+// consecutive rows, so that their loops have one length, 33.4 ms.)  Then
 //   K4(u) = sum over set bits (i, j) of popcount(row_i AND row_j),
 // since row j holds only positions after j.  Vertices with d <= 128 run on
 // one warp (rows of at most 4 words), d <= 512 on a 256-thread CTA, larger
@@ -597,68 +601,160 @@ __device__ __forceinline__ int pos_find(const uint32_t *keys, const uint32_t *po
   }
 }
 
+// The plan's adjacency rows as the kernels read them (rows null: none).
+struct AdjView {
+  const uint32_t *__restrict__ rows;
+  const uint32_t *__restrict__ rowof;
+  const uint32_t *__restrict__ low;
+  uint32_t first, words;
+};
+
+// Columns of the subgraph's bit rows whose ids are among the top ids (positions
+// low .. d - 1 of N+(u)): bit (i, j) is one bit of v_i's adjacency row.  A warp
+// takes a word of columns and 32 rows: lane j keeps where its id lies in an
+// adjacency row, and one load per row and a ballot give the 32 bits, without
+// walking N+(v_i) and looking its ids up.  Work is the pairs of N+(u), not the
+// wedges of u, which are several times as many.
+__device__ __forceinline__ void k4_top_columns(const GraphView &g, const AdjView &adj, const uint32_t *au, uint32_t d,
+                                               uint32_t low, uint32_t W, uint32_t *rows, uint32_t tid, uint32_t nthreads) {
+  const int lane = tid & 31;
+  const uint32_t warp = tid >> 5, warps = nthreads >> 5;
+  const uint32_t w0 = low >> 5;
+  // items (w, rows ib .. ib + 31) with ib <= 32 w + 31: word w has w + 1 blocks
+  // of rows, numbered through all words from w0 on
+  uint32_t w = w0, blk = warp;
+  while (true) {
+    while (w < W && blk > w) {
+      blk -= w + 1;
+      ++w;
+    }
+    if (w >= W) break;
+    const uint32_t j = 32 * w + lane, ib = 32 * blk;
+    const bool col = j >= low && j < d;
+    const uint32_t p = col ? au[j] - adj.first : 0u;
+    const unsigned cols = __ballot_sync(kFull, col);
+    const uint32_t i = ib + lane;
+    uint32_t row = kNoHubRow;
+    if (i < d) {
+      const uint32_t v = au[i];
+      row = v >= adj.first ? v - adj.first : adj.rowof[v];
+    }
+    const unsigned have = __ballot_sync(kFull, row != kNoHubRow);
+    const uint32_t *at = adj.rows + (p >> 5);
+    const uint32_t sh = p & 31u;
+    uint32_t mine = 0;
+#pragma unroll 1
+    for (uint32_t k = 0; k < 32 && ib + k < d; k += 8) {
+      uint32_t x[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const uint32_t r = __shfl_sync(kFull, row, k + q);
+        x[q] = (have >> (k + q)) & 1u ? at[(uint64_t)r * adj.words] : 0u;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const unsigned b = __ballot_sync(kFull, (x[q] >> sh) & 1u) & cols;
+        if (lane == (int)k + q) mine = b;
+      }
+    }
+    if (i < d && mine) atomicOr(&rows[i * W + w], mine);
+    // rows of vertices without an adjacency row: fewer than kAdjMin top ids,
+    // the last of N+(v), each searched among the columns
+    unsigned without = __ballot_sync(kFull, i < d && row == kNoHubRow);
+    if (w == w0 && without) {
+      while (without) {
+        const int k = __ffs(without) - 1;
+        without &= without - 1;
+        const uint2 rv = g.row[au[ib + k]];
+        const uint32_t *av = g.adj + (uint64_t)rv.x * 4;
+        for (uint32_t t = lane; t < rv.y && t < kAdjMin; t += 32) {
+          const uint32_t x = av[rv.y - 1 - t];
+          if (x < adj.first) continue;
+          const uint32_t c = low + prefix_below(au + low, d - low, x);
+          if (c < d && au[c] == x) atomicOr(&rows[(ib + k) * W + (c >> 5)], 1u << (c & 31));
+        }
+      }
+    }
+    blk += warps;
+  }
+}
+
 // 4-cliques with lowest vertex u; `nthreads` threads (one warp or the CTA)
 // cooperate, separated by sync().  On entry and on return every key slot of
 // the hash holds kSentinel and the d * W row words are zero.
 template <typename Sync>
-__device__ unsigned long long k4_vertex(const GraphView &g, uint32_t u, uint32_t *keys, uint32_t *pos,
-                                        uint32_t max_log, uint32_t *rows, uint32_t tid,
+__device__ unsigned long long k4_vertex(const GraphView &g, const AdjView &adj, uint32_t u, uint32_t *keys,
+                                        uint32_t *pos, uint32_t max_log, uint32_t *rows, uint32_t tid,
                                         uint32_t nthreads, Sync sync, unsigned *err) {
   const int lane = tid & 31;
   const uint2 ru = g.row[u];
   const uint32_t d = ru.y;
   const uint32_t *au = g.adj + (uint64_t)ru.x * 4;
   const uint32_t W = (d + 31) >> 5;
-  int l = hash_log2(d);
+  // positions [0, dl) go through the hash, [dl, d) through adjacency rows
+  const uint32_t dl = adj.rows ? adj.low[u] : d;
+  if (dl < d) k4_top_columns(g, adj, au, d, dl, W, rows, tid, nthreads);
+  int l = hash_log2(dl);
   if (l > (int)max_log) l = (int)max_log;
   const uint32_t mask = (1u << l) - 1;
-  const int shift = 32 - l;
-  // at most half the slots: the plan's degree classes keep d there; a list
-  // beyond that (a broken rule) is counted wrongly but reported, never hangs
-  const uint32_t ins = d <= (mask + 1) / 2 ? d : (mask + 1) / 2;
-  if (ins < d && tid == 0) atomicOr(err, kLaunchErrTableFull);
-  for (uint32_t i = tid; i < ins; i += nthreads) pos_insert(keys, pos, mask, shift, au[i], i, err);
-  sync();
-  const uint32_t maxu = au[d - 1];
-  // rows: 32 rows per warp step.  Each N+(v) is read as 32-byte octets from
-  // its (32-byte aligned, padded) start up to the last id <= max N+(u); the
-  // lanes walk the 32 lists' octets flattened.  Ids past that point (larger
-  // ids, padding) are not in N+(u), so the hash rejects them: no mask.
-  const uint4 *adj4 = reinterpret_cast<const uint4 *>(g.adj);
-  auto mark = [&](uint32_t row, uint32_t x) {
-    const int j = pos_find(keys, pos, mask, shift, x);
-    if (j >= 0) atomicOr(&rows[row * W + ((uint32_t)j >> 5)], 1u << (j & 31));
-  };
-  for (uint32_t r0 = tid & ~31u; r0 < d; r0 += nthreads) {
-    const uint32_t i = r0 + lane;
-    uint32_t o0 = 0, no = 0;
-    if (i < d) {
-      const uint2 rv = g.row[au[i]];
-      const uint32_t e = prefix_below(g.adj + (uint64_t)rv.x * 4, rv.y, maxu + 1);  // ids <= max N+(u)
-      o0 = rv.x >> 1;
-      no = (e + 7) >> 3;
-    }
-    const uint32_t incl = warp_inclusive_sum(no, lane);
-    const uint32_t total = __shfl_sync(kFull, incl, 31);
-    const uint32_t bias = o0 - (incl - no);
-    WarpRuns own(incl - no, no, lane);
-    for (uint32_t pb = 0; pb < total; pb += 32) {
-      const uint32_t p = pb + lane;
-      const int o = (int)own.owner(pb);
-      const uint32_t oc = __shfl_sync(kFull, bias, o) + p;
-      if (p < total) {
-        const uint4 a = adj4[2 * (uint64_t)oc], b = adj4[2 * (uint64_t)oc + 1];
-        const uint32_t row = r0 + o;
-        mark(row, a.x); mark(row, a.y); mark(row, a.z); mark(row, a.w);
-        mark(row, b.x); mark(row, b.y); mark(row, b.z); mark(row, b.w);
+  if (dl > 1) {
+    const int shift = 32 - l;
+    // at most half the slots: the plan's degree classes keep d there; a list
+    // beyond that (a broken rule) is counted wrongly but reported, never hangs
+    const uint32_t ins = dl <= (mask + 1) / 2 ? dl : (mask + 1) / 2;
+    if (ins < dl && tid == 0) atomicOr(err, kLaunchErrTableFull);
+    for (uint32_t i = tid; i < ins; i += nthreads) pos_insert(keys, pos, mask, shift, au[i], i, err);
+    sync();
+    const uint32_t maxu = au[dl - 1];
+    // rows: 32 rows per warp step.  Each N+(v) is read as 32-byte octets from
+    // its (32-byte aligned, padded) start up to the last id <= the last hashed
+    // one; the lanes walk the 32 lists' octets flattened.  Ids past that point
+    // (larger ids, padding) are not in the hash, which rejects them: no mask.
+    const uint4 *adj4 = reinterpret_cast<const uint4 *>(g.adj);
+    auto mark = [&](uint32_t row, uint32_t x) {
+      const int j = pos_find(keys, pos, mask, shift, x);
+      if (j >= 0) atomicOr(&rows[row * W + ((uint32_t)j >> 5)], 1u << (j & 31));
+    };
+    for (uint32_t r0 = tid & ~31u; r0 < dl; r0 += nthreads) {
+      const uint32_t i = r0 + lane;
+      uint32_t o0 = 0, no = 0;
+      if (i < dl) {
+        const uint2 rv = g.row[au[i]];
+        const uint32_t e = prefix_below(g.adj + (uint64_t)rv.x * 4, rv.y, maxu + 1);  // ids <= maxu
+        o0 = rv.x >> 1;
+        no = (e + 7) >> 3;
+      }
+      const uint32_t incl = warp_inclusive_sum(no, lane);
+      const uint32_t total = __shfl_sync(kFull, incl, 31);
+      const uint32_t bias = o0 - (incl - no);
+      WarpRuns own(incl - no, no, lane);
+      for (uint32_t pb = 0; pb < total; pb += 32) {
+        const uint32_t p = pb + lane;
+        const int o = (int)own.owner(pb);
+        const uint32_t oc = __shfl_sync(kFull, bias, o) + p;
+        if (p < total) {
+          const uint4 a = adj4[2 * (uint64_t)oc], b = adj4[2 * (uint64_t)oc + 1];
+          const uint32_t row = r0 + o;
+          mark(row, a.x); mark(row, a.y); mark(row, a.z); mark(row, a.w);
+          mark(row, b.x); mark(row, b.y); mark(row, b.z); mark(row, b.w);
+        }
       }
     }
   }
   sync();
-  // count: for every set bit (i, j), the common later positions of rows i and j
+  // count: for every set bit (i, j), the common later positions of rows i and
+  // j.  The lanes of a warp take one word of consecutive rows, so that their
+  // inner loops have the same length; word w has bits in rows up to 32 w + 30 only.
   unsigned long long cnt = 0;
-  for (uint32_t it = tid; it < d * W; it += nthreads) {
-    const uint32_t i = it / W, w = it - i * W;
+  uint32_t i = tid, w = 0;
+  while (true) {
+    uint32_t nr = min(d, 32 * w + 31);
+    while (w < W && i >= nr) {
+      i -= nr;
+      ++w;
+      nr = min(d, 32 * w + 31);
+    }
+    if (w >= W) break;
     const uint32_t *ri = rows + i * W;
     uint32_t bits = ri[w];
     while (bits) {
@@ -667,10 +763,12 @@ __device__ unsigned long long k4_vertex(const GraphView &g, uint32_t u, uint32_t
       const uint32_t *rj = rows + j * W;
       for (uint32_t ww = w; ww < W; ++ww) cnt += __popc(ri[ww] & rj[ww]);
     }
+    i += nthreads;
   }
   sync();
   for (uint32_t it = tid; it < d * W; it += nthreads) rows[it] = 0;
-  for (uint32_t h = tid; h <= mask; h += nthreads) keys[h] = kSentinel;
+  if (dl > 1)
+    for (uint32_t h = tid; h <= mask; h += nthreads) keys[h] = kSentinel;
   sync();
   return cnt;
 }
@@ -679,7 +777,7 @@ __device__ unsigned long long k4_vertex(const GraphView &g, uint32_t u, uint32_t
 // every vertex keeps its rows in its CTA's HBM buffer, and the CTA holds only
 // the position hash in shared memory.
 template <int THREADS, int HLOG, uint32_t ROWW>
-__device__ __forceinline__ void k4_cta_body(GraphView g, const uint32_t *__restrict__ list, uint32_t lo,
+__device__ __forceinline__ void k4_cta_body(GraphView g, AdjView adj, const uint32_t *__restrict__ list, uint32_t lo,
                                             uint32_t hi, uint32_t *__restrict__ pool, uint64_t pool_words,
                                             uint32_t *counter, unsigned *err,
                                             unsigned long long *__restrict__ out) {
@@ -699,7 +797,7 @@ __device__ __forceinline__ void k4_cta_body(GraphView g, const uint32_t *__restr
     const uint32_t d = g.row[u].y;
     const uint64_t words = (uint64_t)d * ((d + 31) >> 5);
     uint32_t *rows = words <= ROWW ? srows : pool + (uint64_t)blockIdx.x * pool_words;
-    cnt += k4_vertex(g, u, keys, pos, HLOG, rows, threadIdx.x, blockDim.x, [] { __syncthreads(); }, err);
+    cnt += k4_vertex(g, adj, u, keys, pos, HLOG, rows, threadIdx.x, blockDim.x, [] { __syncthreads(); }, err);
   }
   cnt = warp_sum_u64(cnt);
   if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(out, cnt);
@@ -707,24 +805,24 @@ __device__ __forceinline__ void k4_cta_body(GraphView g, const uint32_t *__restr
 
 template <int THREADS, int HLOG, uint32_t ROWW>
 __global__ void __launch_bounds__(THREADS)
-    k_k4_cta(GraphView g, const uint32_t *__restrict__ list, uint32_t lo, uint32_t hi,
+    k_k4_cta(GraphView g, AdjView adj, const uint32_t *__restrict__ list, uint32_t lo, uint32_t hi,
              uint32_t *__restrict__ pool, uint64_t pool_words, uint32_t *counter, unsigned *err,
              unsigned long long *__restrict__ out) {
-  k4_cta_body<THREADS, HLOG, ROWW>(g, list, lo, hi, pool, pool_words, counter, err, out);
+  k4_cta_body<THREADS, HLOG, ROWW>(g, adj, list, lo, hi, pool, pool_words, counter, err, out);
 }
 
 // Vertices whose rows live in HBM: two 1024-thread CTAs share an SM.
 __global__ void __launch_bounds__(kK4BigThreads, kK4PoolPerSm)
-    k_k4_pool(GraphView g, const uint32_t *__restrict__ list, uint32_t lo, uint32_t hi,
+    k_k4_pool(GraphView g, AdjView adj, const uint32_t *__restrict__ list, uint32_t lo, uint32_t hi,
               uint32_t *__restrict__ pool, uint64_t pool_words, uint32_t *counter, unsigned *err,
               unsigned long long *__restrict__ out) {
-  k4_cta_body<kK4BigThreads, kK4PoolLog, 0>(g, list, lo, hi, pool, pool_words, counter, err, out);
+  k4_cta_body<kK4BigThreads, kK4PoolLog, 0>(g, adj, list, lo, hi, pool, pool_words, counter, err, out);
 }
 
 // Warp vertices: each warp in its own region of shared memory, one vertex per
 // claim (32 per claim left a tail of costly vertices: RMAT-22 129.1 -> 119.6 ms).
 __global__ void __launch_bounds__(kK4WarpCtaWarps * 32)
-    k_k4_warp(GraphView g, const uint32_t *__restrict__ list, uint32_t lo, uint32_t hi,
+    k_k4_warp(GraphView g, AdjView adj, const uint32_t *__restrict__ list, uint32_t lo, uint32_t hi,
               uint32_t *counter, unsigned *err, unsigned long long *__restrict__ out) {
   extern __shared__ __align__(16) uint32_t sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -739,7 +837,7 @@ __global__ void __launch_bounds__(kK4WarpCtaWarps * 32)
     if (lane == 0) c = atomicAdd(counter, 1u);
     c = __shfl_sync(kFull, c, 0);
     if (lo + c >= hi) break;
-    cnt += k4_vertex(g, list[lo + c], keys, pos, kK4WarpLog, rows, lane, 32, [] { __syncwarp(); }, err);
+    cnt += k4_vertex(g, adj, list[lo + c], keys, pos, kK4WarpLog, rows, lane, 32, [] { __syncwarp(); }, err);
   }
   cnt = warp_sum_u64(cnt);
   if (lane == 0 && cnt) atomicAdd(out, cnt);
@@ -890,6 +988,7 @@ int build_k4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
   ScratchAlloc pol_alloc{s};
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
   const uint32_t *dp = g->dag.outdeg.p;
+  GARY_TRY(build_adj_rows(g, s, plan->adj));
   // warp and mid vertices in id order; big vertices largest first
   GARY_TRY(plan->light.alloc_persistent(std::max<uint32_t>(n, 1)));
   plan->n_light = (uint32_t)(thrust::copy_if(pol, thrust::counting_iterator<uint32_t>(0),
@@ -967,6 +1066,8 @@ int launch_k4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaS
   GARY_CUDA(cudaMemsetAsync(d_out, 0, 8, s));
   GARY_CUDA(cudaEventRecord(g->ev0, s));
   const GraphView gv = g->view();
+  const AdjView av{plan->adj.words ? reinterpret_cast<const uint32_t *>(plan->adj.rows.p) : nullptr, plan->adj.rowof.p,
+                   plan->adj.low.p, plan->adj.first, plan->adj.words};
   // The HBM-row vertices are the largest: their kernel runs first.
   if (p1 > p0) {
     // rows in HBM: the pool holds one row buffer per CTA of the grid
@@ -975,18 +1076,18 @@ int launch_k4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaS
       set_error("4-clique row pool missing for %u vertices", p1 - p0);
       return GARY_ERR_INVALID;
     }
-    pool<<<grid, kK4BigThreads, smem_pool, s>>>(gv, plan->big.p, p0, p1, plan->cursors.p, pool_words,
+    pool<<<grid, kK4BigThreads, smem_pool, s>>>(gv, av, plan->big.p, p0, p1, plan->cursors.p, pool_words,
                                                 &st->next_cta, &st->error, d_out);
   }
   if (b1 > b0)  // rows in shared memory, two CTAs per SM
     big<<<std::min<unsigned>((unsigned)(sm_count() * per_big), b1 - b0), kK4BigThreads, smem_big, s>>>(
-        gv, plan->big.p, b0, b1, nullptr, 0, &st->next_big, &st->error, d_out);
+        gv, av, plan->big.p, b0, b1, nullptr, 0, &st->next_big, &st->error, d_out);
   if (m1 > m0)
     mid<<<std::min<unsigned>((unsigned)(sm_count() * per_mid), m1 - m0), kK4MidThreads, smem_mid, s>>>(
-        gv, plan->mid.p, m0, m1, nullptr, 0, &st->next_aux, &st->error, d_out);
+        gv, av, plan->mid.p, m0, m1, nullptr, 0, &st->next_aux, &st->error, d_out);
   if (w1 > w0)
     k_k4_warp<<<(unsigned)(sm_count() * per_warp), kK4WarpCtaWarps * 32, smem_warp, s>>>(
-        gv, plan->light.p, w0, w1, &st->next_warp, &st->error, d_out);
+        gv, av, plan->light.p, w0, w1, &st->next_warp, &st->error, d_out);
   GARY_CUDA(cudaGetLastError());
   GARY_CUDA(cudaEventRecord(g->ev1, s));
   g->last = gary_count_stats{};
