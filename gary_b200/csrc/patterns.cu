@@ -561,8 +561,8 @@ __global__ void __launch_bounds__(kWinThreads, 3)
 //   warp vertices (3 <= d+ <= 128): one warp each, 8-warp CTAs, several per SM;
 //   mid vertices (128 < d+ <= 362): a 256-thread CTA each, rows in 17 KiB of
 //     shared memory, eight CTAs per SM (one waits at a barrier, others run);
-//   big vertices (d+ > 362): a 1024-thread CTA each, two per SM: rows in 96
-//     KiB of shared memory up to d+ = 877; beyond, rows in a per-CTA HBM buffer
+//   big vertices (d+ > 362): a CTA each, two per SM: 512 threads with rows in 96
+//     KiB of shared memory up to d+ = 877; beyond, 1024 threads and rows in a per-CTA HBM buffer
 //     and only the position hash in shared memory (k_k4_pool, run first: its
 //     vertices are the largest).
 // (class bounds, table sizes and row words: pattern_rules.cuh)
@@ -570,6 +570,10 @@ constexpr uint32_t kK4WarpWords = 1024;       // shared words per warp: 32 KiB p
 constexpr int kK4WarpCtaWarps = 8;
 constexpr int kK4MidThreads = 256;
 constexpr int kK4BigThreads = 1024;
+// Shared-row vertices: two CTAs of 512 threads per SM, one at a barrier while
+// the other runs.  Of 1024 threads at the 40 registers the kernel takes only
+// one fits (RMAT-22 ef16, ms a count: 256 / 512 / 1024 threads 33.9 / 31.2 / 33.3).
+constexpr int kK4SharedThreads = 512;
 constexpr uint32_t kK4PoolPerSm = 2;         // CTAs per SM of the HBM-row kernel
 static_assert(2 * (1u << kK4WarpLog) + kK4WarpRowWords <= kK4WarpWords, "warp region too small");
 
@@ -1033,7 +1037,7 @@ int launch_k4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaS
   const uint32_t b0 = np + part(ns, shard), b1 = np + part(ns, shard + 1);
   const uint32_t m0 = part(plan->n_mid, shard), m1 = part(plan->n_mid, shard + 1);
   const uint32_t w0 = part(plan->n_light, shard), w1 = part(plan->n_light, shard + 1);
-  auto big = k_k4_cta<kK4BigThreads, kK4BigLog, kK4BigRowWords>;
+  auto big = k_k4_cta<kK4SharedThreads, kK4BigLog, kK4BigRowWords>;
   auto pool = k_k4_pool;
   const size_t smem_pool = 2 * (1u << kK4PoolLog) * 4;
   auto mid = k_k4_cta<kK4MidThreads, kK4MidLog, kK4MidRowWords>;
@@ -1050,7 +1054,7 @@ int launch_k4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaS
     attr[dev] = true;
   }
   int per_mid = 0, per_warp = 0, per_pool = 0, per_big = 0;
-  GARY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_big, big, kK4BigThreads, smem_big));
+  GARY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_big, big, kK4SharedThreads, smem_big));
   per_big = std::max(per_big, 1);
   GARY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_pool, pool, kK4BigThreads, smem_pool));
   per_pool = std::max(per_pool, 1);
@@ -1080,7 +1084,7 @@ int launch_k4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaS
                                                 &st->next_cta, &st->error, d_out);
   }
   if (b1 > b0)  // rows in shared memory, two CTAs per SM
-    big<<<std::min<unsigned>((unsigned)(sm_count() * per_big), b1 - b0), kK4BigThreads, smem_big, s>>>(
+    big<<<std::min<unsigned>((unsigned)(sm_count() * per_big), b1 - b0), kK4SharedThreads, smem_big, s>>>(
         gv, av, plan->big.p, b0, b1, nullptr, 0, &st->next_big, &st->error, d_out);
   if (m1 > m0)
     mid<<<std::min<unsigned>((unsigned)(sm_count() * per_mid), m1 - m0), kK4MidThreads, smem_mid, s>>>(
