@@ -192,7 +192,8 @@ def workload_config(args, world: int) -> dict:
 # profiles/ applies to the build whose sources hash to its "kernel_src".
 KERNEL_SOURCES = ("tc.cu", "tc.cuh", "hub.cu", "hub.cuh", "pair_set.cuh", "warp_ops.cuh", "bulk.cuh", "internal.cuh", "graph.cuh")
 # the 4-cycle and 4-clique count kernels
-PATTERN_SOURCES = ("patterns.cu", "patterns.cuh", "hub.cu", "hub.cuh", "pattern_rules.cuh", "warp_ops.cuh", "internal.cuh", "graph.cuh")
+PATTERN_SOURCES = ("patterns.cu", "patterns.cuh", "c4_rows.cu", "c4_rows.cuh", "hub.cu", "hub.cuh",
+                   "pattern_rules.cuh", "warp_ops.cuh", "internal.cuh", "graph.cuh")
 
 
 def kernel_source_hash(sources=KERNEL_SOURCES) -> str:

@@ -855,12 +855,12 @@ struct ClassIs {
 };
 // C4 per-vertex class by an upper bound of its wedge count.
 __global__ void k_c4_classify(const uint2 *__restrict__ srow, const uint32_t *__restrict__ sadj,
-                              const uint32_t *__restrict__ dplus, uint32_t n, uint32_t warp_cap,
+                              const uint32_t *__restrict__ dplus, uint32_t n, uint32_t lowest, uint32_t warp_cap,
                               uint8_t *__restrict__ cls) {
   for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n;
        u += (uint64_t)gridDim.x * blockDim.x) {
     const uint2 r = srow[u];
-    const uint32_t pre = r.y - dplus[u];
+    const uint32_t pre = u < lowest ? r.y - dplus[u] : 0u;  // the vertices above are counted by rows
     uint64_t w = 0;
     for (uint32_t k = 0; k < pre && w <= warp_cap; ++k) w += srow[sadj[(uint64_t)r.x * 4 + k]].y;
     // w: the wedge bound, its sum stopped once past the light limit; the
@@ -1111,7 +1111,8 @@ int build_c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
   DevBuf<uint8_t> cls;
   GARY_TRY(cls.alloc(n, s));
-  k_c4_classify<<<grid_for(n), kThreads, 0, s>>>(g->sym.row.p, g->sym.adj.p, g->dag.outdeg.p, n,
+  GARY_TRY(build_c4_rows(g, s, plan->rows));
+  k_c4_classify<<<grid_for(n), kThreads, 0, s>>>(g->sym.row.p, g->sym.adj.p, g->dag.outdeg.p, n, plan->rows.lowest,
                                                  (uint32_t)kC4LightWedges, cls.p);
   GARY_CUDA(cudaGetLastError());
   GARY_TRY(plan->light.alloc_persistent(std::max<uint32_t>(n, 1)));
@@ -1210,6 +1211,7 @@ int launch_c4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaS
   GARY_CUDA(cudaMemsetAsync(plan->sched.p, 0, sizeof(SchedState), s));
   GARY_CUDA(cudaMemsetAsync(d_out, 0, 8, s));
   GARY_CUDA(cudaEventRecord(g->ev0, s));
+  GARY_TRY(launch_c4_rows(g, plan->rows, d_out, s, shard, nshards));
   if (t1 > t0)
     k_c4_win<<<std::min<uint32_t>(plan->win_ctas, t1 - t0), kWinThreads, smem_win, s>>>(
         sv, plan->tiles.p, t0, t1, plan->cursors.p, std::max(plan->max_pre, 1u), plan->sched.p, d_out);

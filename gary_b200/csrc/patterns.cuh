@@ -2,6 +2,7 @@
 #pragma once
 #include <cstdint>
 
+#include "c4_rows.cuh"
 #include "graph.cuh"
 #include "hub.cuh"
 #include "pattern_rules.cuh"
@@ -18,6 +19,7 @@ struct PatternPlan {
   DevBuf<uint32_t> big;      // K4: vertices with d+ > 512, largest first (the n_pool with rows in HBM first)
   DevBuf<uint32_t> cursors;  // C4: per window-kernel CTA, 6 x max_pre words of list state; K4: row pool
   AdjRows adj;               // K4: adjacency rows over the top ids
+  C4Rows rows;               // C4: the vertices u counted by rows
   DevBuf<SchedState> sched;
   uint32_t n_cta = 0, n_warp = 0, n_light = 0, n_mid = 0, n_big = 0, n_pool = 0, max_pre = 0, win_ctas = 0;
 };
