@@ -21,6 +21,11 @@ constexpr uint64_t kC4LightWedges = kC4WarpSlots / 2;
 // vertex's wedge count, since each v adds at most one to it.
 constexpr uint32_t kC4MidSlots = 16384;
 constexpr uint64_t kC4MidWedges = kC4MidSlots / 2;
+// Those of at most kC4Mid1Wedges wedges get a smaller map of their own (its
+// CTAs are smaller, and many more of them share an SM); every map's part in use
+// is sized by the vertex's own wedge count, at most half full.
+constexpr uint32_t kC4Mid1Slots = 4096;
+constexpr uint64_t kC4Mid1Wedges = kC4Mid1Slots / 2;
 // Heavy vertices count in windows: 16-bit counters while c(u, w) <= the
 // number of lower neighbours fits, 32-bit ones (half windows) beyond.
 constexpr uint32_t kC4Win16MaxPre = 0xFFFFu;

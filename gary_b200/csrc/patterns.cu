@@ -93,8 +93,10 @@ __device__ __forceinline__ uint32_t below_u(const uint32_t *l, uint32_t len, uin
 }
 
 // Walk every wedge u - v - w with v in N(u), v < u, and w in N(v), w < u,
-// for v = N(u)[k], k in the 32-wide steps kb, kb + kstep, ... < ke; call
-// f(w) for each.  All 32 lanes must call.
+// for v = N(u)[k], k in the 32-wide steps kb, kb + kstep, ... < ke; call f on
+// the quads of the lists they lie in, in all lanes together: the ids of a quad
+// that are not below u (ids past the run, padding, lanes without a quad) are no
+// wedge ends.  All 32 lanes must call.
 template <typename F>
 __device__ __forceinline__ void c4_wedges(const GraphView &s, const uint32_t *__restrict__ dplus,
                                           const uint32_t *__restrict__ au, uint32_t u, uint32_t kb,
@@ -122,39 +124,71 @@ __device__ __forceinline__ void c4_wedges(const GraphView &s, const uint32_t *__
       const uint32_t qi = __shfl_sync(kFull, qbase, o) + p;
       return p < total ? adj4[qi] : make_uint4(kSentinel, kSentinel, kSentinel, kSentinel);
     };
-    auto take = [&](const uint4 &a) {
-      if (a.x < u) f(a.x);
-      if (a.y < u) f(a.y);
-      if (a.z < u) f(a.z);
-      if (a.w < u) f(a.w);
-    };
     uint4 cur = fetch(0);
     for (uint32_t pb = 32; pb < total; pb += 32) {
       const uint4 nxt = fetch(pb);
-      take(cur);
+      f(cur);
       cur = nxt;
     }
-    take(cur);
+    f(cur);
   }
 }
 
-// Counter map in shared memory: increments c(w) and returns the old value.
-// The plan keeps the map at most half full; a probe that finds every slot
-// taken (a broken capacity rule) sets kLaunchErrTableFull and counts nothing.
-__device__ __forceinline__ uint32_t map_incr(uint32_t *keys, uint32_t *vals, uint32_t mask, int shift,
-                                             uint32_t w, unsigned *err) {
-  uint32_t h = (w * kHashMul) >> shift;
-  for (uint32_t i = 0; i <= mask; ++i) {
-    const uint32_t k = keys[h];
-    if (k == w) return atomicAdd(&vals[h], 1u);
-    if (k == kSentinel) {
-      const uint32_t old = atomicCAS(&keys[h], kSentinel, w);
-      if (old == kSentinel || old == w) return atomicAdd(&vals[h], 1u);
-    }
-    h = (h + 1) & mask;
+// Counter map in shared memory: the ids of a quad that lie in [lo, lo + span)
+// are counted, and the sum of their counters' old values returned.  WIDE: 32-bit
+// counters, one a slot; else 16-bit ones, slot h's in half h & 1 of word h / 2.
+// The four first probes are loads in flight together, and most ids are settled
+// by them; the others probe on one after the other, the warp meeting again after
+// each, so that the counters' increments run with all lanes (one divergent
+// insert-and-count loop per id left a lane or two active at a time).  The plan
+// keeps the map at most half full; a probe that finds every slot taken (a broken
+// capacity rule) sets kLaunchErrTableFull and counts nothing.  All 32 lanes call.
+template <bool WIDE>
+__device__ __forceinline__ uint32_t map_incr4(uint32_t *keys, uint32_t *vals, uint32_t mask, int shift, const uint4 &a,
+                                              uint32_t lo, uint32_t span, unsigned *err) {
+  const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+  uint32_t h[4], k[4];
+  bool on[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    on[j] = w[j] - lo < span;
+    h[j] = (w[j] * kHashMul) >> shift;
+    k[j] = keys[h[j]];
   }
-  atomicOr(err, kLaunchErrTableFull);
-  return 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (on[j] && k[j] != w[j]) {
+      uint32_t x = k[j], at = h[j];
+      for (uint32_t i = 0;; ++i) {
+        if (x == kSentinel) {
+          x = atomicCAS(&keys[at], kSentinel, w[j]);
+          if (x == kSentinel) break;
+        }
+        if (x == w[j]) break;
+        if (i > mask) {
+          atomicOr(err, kLaunchErrTableFull);
+          on[j] = false;
+          break;
+        }
+        at = (at + 1) & mask;
+        x = keys[at];
+      }
+      h[j] = at;
+    }
+    __syncwarp();
+  }
+  uint32_t sum = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (!on[j]) continue;
+    if (WIDE) {
+      sum += atomicAdd(&vals[h[j]], 1u);
+    } else {
+      const uint32_t sh = (h[j] & 1u) << 4;
+      sum += (atomicAdd(&vals[h[j] >> 1], 1u << sh) >> sh) & 0xFFFFu;
+    }
+  }
+  return sum;
 }
 
 __global__ void __launch_bounds__(kPWarps * 32)
@@ -177,13 +211,18 @@ __global__ void __launch_bounds__(kPWarps * 32)
       const uint2 ru = s.row[u];
       const uint32_t pre = ru.y - dplus[u];  // neighbours ranked below u
       const uint32_t *au = s.adj + (uint64_t)ru.x * 4;
-      for (uint32_t i = lane; i < kPSlots; i += 32) {
+      // the part of the map in use: at least two slots a wedge
+      uint32_t bound = 0;
+      for (uint32_t k = lane; k < pre; k += 32) bound += s.row[au[k]].y;
+      const int log = min(hash_log2(__reduce_add_sync(kFull, bound)), 10);
+      const uint32_t slots = 1u << log;
+      for (uint32_t i = lane; i < slots; i += 32) {
         keys[i] = kSentinel;
         vals[i] = 0;
       }
       __syncwarp();
-      c4_wedges(s, dplus, au, u, 0, pre, 32, lane, [&](uint32_t w) {
-        acc += map_incr(keys, vals, kPSlots - 1, 32 - 10, w, &sched->error);
+      c4_wedges(s, dplus, au, u, 0, pre, 32, lane, [&](const uint4 &a) {
+        acc += map_incr4<true>(keys, vals, slots - 1, 32 - log, a, 0, u, &sched->error);
       });
       __syncwarp();
     }
@@ -195,69 +234,63 @@ __global__ void __launch_bounds__(kPWarps * 32)
 // ---- C4, medium vertices: one CTA-wide shared hash map per vertex ---------
 // A count c(u,w) never exceeds the vertex's wedge count (each v adds at most
 // one to it), at most kMidWedges here, so counts are 16 bits, two to a word:
-// keys 64 KiB + counts 32 KiB, and two CTAs share an SM.
-constexpr uint32_t kMidSlots = kC4MidSlots;
-constexpr int kMidLog = 14;
-static_assert((1u << kMidLog) == kMidSlots, "medium map size");
-constexpr int kMidThreads = 512;
+// keys 64 KiB + counts 32 KiB, and two 512-thread CTAs share an SM.  Vertices of
+// up to kC4Mid1Wedges wedges run 128-thread CTAs with a quarter of the map, eight
+// per SM: they have a few dozen lower neighbours, a warp's worth, and time goes
+// in the chain of dependent loads, not in threads (RMAT-22 ef16: 13.7 ms for
+// 66 K medium vertices in 512-thread CTAs that cleared the whole map each time).
+constexpr int kMidLog = 14, kMid1Log = 12;
+static_assert((1u << kMidLog) == kC4MidSlots && (1u << kMid1Log) == kC4Mid1Slots, "medium map sizes");
+constexpr int kMidThreads = 512, kMid1Threads = 128;
 constexpr uint64_t kMidWedges = kC4MidWedges;  // wedges (>= distinct w) a medium vertex may have
-constexpr uint32_t kMidWords = kMidSlots + kMidSlots / 2;
+constexpr uint32_t mid_words(int log) { return (1u << log) + (1u << log) / 2; }
 static_assert(kMidWedges < 65536, "16-bit medium counts");
 
-// As map_incr, with the count of slot h in half h & 1 of word h / 2 of vals2.
-__device__ __forceinline__ uint32_t map_incr16(uint32_t *keys, uint32_t *vals2, uint32_t mask, int shift,
-                                               uint32_t w, unsigned *err) {
-  uint32_t h = (w * kHashMul) >> shift;
-  for (uint32_t i = 0; i <= mask; ++i) {
-    const uint32_t k = keys[h];
-    bool hit = k == w;
-    if (!hit && k == kSentinel) {
-      const uint32_t old = atomicCAS(&keys[h], kSentinel, w);
-      hit = old == kSentinel || old == w;
-    }
-    if (hit) {
-      const uint32_t sh = (h & 1u) << 4;
-      return (atomicAdd(&vals2[h >> 1], 1u << sh) >> sh) & 0xFFFFu;
-    }
-    h = (h + 1) & mask;
-  }
-  atomicOr(err, kLaunchErrTableFull);
-  return 0;
+// Lower neighbours a warp takes at a time: some four claims per warp of the
+// CTA.  Claims of 32 left most of 16 warps waiting at the barrier for the few
+// that had one (pre is about 110 for a medium vertex at RMAT-22).
+__device__ __forceinline__ uint32_t claim_size(uint32_t pre, uint32_t warps) {
+  return min(max(pre / (4u * warps), 4u), 32u);
 }
 
-__global__ void __launch_bounds__(kMidThreads, 2)
+template <int THREADS, int LOG, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB)
     k_c4_mid(GraphView s, const uint32_t *__restrict__ dplus, const uint32_t *__restrict__ mid,
-             uint32_t n_mid, SchedState *sched, unsigned long long *__restrict__ out) {
+             const uint32_t *__restrict__ wed, uint32_t n_mid, uint32_t *next, unsigned *err,
+             unsigned long long *__restrict__ out) {
   extern __shared__ __align__(16) uint32_t sm[];
-  uint32_t *keys = sm, *vals = sm + kMidSlots;  // vals: kMidSlots / 2 words of 16-bit pairs
+  uint32_t *keys = sm, *vals = sm + (1u << LOG);  // vals: half as many words, of 16-bit pairs
   __shared__ uint32_t s_u, s_next;
   const int lane = threadIdx.x & 31;
   unsigned long long acc = 0;
-  for (uint32_t i = threadIdx.x; i < kMidSlots; i += blockDim.x) keys[i] = kSentinel;
-  for (uint32_t i = threadIdx.x; i < kMidSlots / 2; i += blockDim.x) vals[i] = 0;
+  for (uint32_t i = threadIdx.x; i < (1u << LOG); i += THREADS) keys[i] = kSentinel;
+  for (uint32_t i = threadIdx.x; i < (1u << LOG) / 2; i += THREADS) vals[i] = 0;
   while (true) {
     if (threadIdx.x == 0) {
-      s_u = atomicAdd(&sched->next_aux, 1u);
+      s_u = atomicAdd(next, 1u);
       s_next = 0;
     }
     __syncthreads();
-    if (s_u >= n_mid) break;
-    const uint32_t u = mid[s_u];
+    const uint32_t i = s_u;
+    if (i >= n_mid) break;
+    const uint32_t u = mid[i];
+    const int log = min(hash_log2(wed[i]), LOG);  // the part of the map in use
     const uint2 ru = s.row[u];
     const uint32_t pre = ru.y - dplus[u];
     const uint32_t *au = s.adj + (uint64_t)ru.x * 4;
+    const uint32_t grab = claim_size(pre, THREADS / 32);
     while (true) {
       uint32_t k = 0;
-      if (lane == 0) k = atomicAdd(&s_next, 32u);
+      if (lane == 0) k = atomicAdd(&s_next, grab);
       k = __shfl_sync(kFull, k, 0);
       if (k >= pre) break;
-      c4_wedges(s, dplus, au, u, k, min(k + 32, pre), 32, lane, [&](uint32_t w) {
-        acc += map_incr16(keys, vals, kMidSlots - 1, 32 - kMidLog, w, &sched->error);
+      c4_wedges(s, dplus, au, u, k, min(k + grab, pre), 32, lane, [&](const uint4 &a) {
+        acc += map_incr4<false>(keys, vals, (1u << log) - 1, 32 - log, a, 0, u, err);
       });
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < kMidSlots; i += blockDim.x) keys[i] = kSentinel;
-    for (uint32_t i = threadIdx.x; i < kMidSlots / 2; i += blockDim.x) vals[i] = 0;
+    for (uint32_t h = threadIdx.x; h < (1u << log); h += THREADS) keys[h] = kSentinel;
+    for (uint32_t h = threadIdx.x; h < (1u << log) / 2; h += THREADS) vals[h] = 0;
     // the loop head's barrier orders this reset before the next vertex
   }
   acc = warp_sum_u64(acc);
@@ -952,13 +985,18 @@ struct DegOf {
   const uint32_t *d;
   __host__ __device__ uint32_t operator()(uint32_t u) const { return d[u]; }
 };
-struct AtMost {
-  uint64_t cap;
-  __host__ __device__ bool operator()(uint64_t w) const { return w <= cap; }
+// Workers of the vertices beyond the light ones.
+enum C4Worker : uint8_t { kC4WMid1 = 1, kC4WMid = 2, kC4WHeavy = 3 };
+__global__ void k_c4_workers(const uint64_t *__restrict__ wed, uint32_t nl, uint8_t *__restrict__ worker) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nl; i += (uint64_t)gridDim.x * blockDim.x)
+    worker[i] = wed[i] <= kC4Mid1Wedges ? kC4WMid1 : wed[i] <= kC4MidWedges ? kC4WMid : kC4WHeavy;
+}
+struct IsWorker {
+  uint8_t w;
+  __host__ __device__ bool operator()(uint8_t x) const { return x == w; }
 };
-struct Above {
-  uint64_t cap;
-  __host__ __device__ bool operator()(uint64_t w) const { return w > cap; }
+struct ToU32 {
+  __host__ __device__ uint32_t operator()(uint64_t x) const { return (uint32_t)x; }
 };
 struct PreOf {
   const uint2 *srow;
@@ -1132,14 +1170,25 @@ int build_c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
                                                                        g->dag.outdeg.p, big.p, nb, wed.p);
     GARY_CUDA(cudaGetLastError());
   }
+  DevBuf<uint8_t> worker;
+  GARY_TRY(worker.alloc(std::max<uint32_t>(nb, 1), s));
+  if (nb) k_c4_workers<<<grid_for(nb), kThreads, 0, s>>>(wed.p, nb, worker.p);
+  GARY_CUDA(cudaGetLastError());
+  auto pick = [&](uint32_t *to, uint8_t w) {
+    return (uint32_t)(thrust::copy_if(pol, big.p, big.p + nb, worker.p, to, IsWorker{w}) - to);
+  };
+  auto wed32 = thrust::make_transform_iterator(wed.p, ToU32{});  // medium wedge counts fit
+  auto pick_wed = [&](uint32_t *to, uint8_t w) { thrust::copy_if(pol, wed32, wed32 + nb, worker.p, to, IsWorker{w}); };
   GARY_TRY(plan->mid.alloc_persistent(std::max<uint32_t>(nb, 1)));
-  plan->n_mid = (uint32_t)(thrust::copy_if(pol, big.p, big.p + nb, wed.p, plan->mid.p,
-                                           AtMost{kMidWedges}) - plan->mid.p);
+  GARY_TRY(plan->mid_wed.alloc_persistent(std::max<uint32_t>(nb, 1)));
+  plan->n_mid1 = pick(plan->mid.p, kC4WMid1);
+  plan->n_mid = plan->n_mid1 + pick(plan->mid.p + plan->n_mid1, kC4WMid);
+  pick_wed(plan->mid_wed.p, kC4WMid1);
+  pick_wed(plan->mid_wed.p + plan->n_mid1, kC4WMid);
   DevBuf<uint32_t> heavy;
   DevBuf<uint64_t> cost;
   GARY_TRY(heavy.alloc(std::max<uint32_t>(nb, 1), s));
-  const uint32_t nh = (uint32_t)(thrust::copy_if(pol, big.p, big.p + nb, wed.p, heavy.p,
-                                                 Above{kMidWedges}) - heavy.p);
+  const uint32_t nh = pick(heavy.p, kC4WHeavy);
   GARY_TRY(cost.alloc(std::max<uint32_t>(nh, 1), s));
   GARY_TRY(c4_win_attr());
   {
@@ -1151,7 +1200,7 @@ int build_c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
   if (nh) {
     DevBuf<uint64_t> hw;
     GARY_TRY(hw.alloc(nh, s));
-    thrust::copy_if(pol, wed.p, wed.p + nb, wed.p, hw.p, Above{kMidWedges});
+    thrust::copy_if(pol, wed.p, wed.p + nb, worker.p, hw.p, IsWorker{kC4WHeavy});
     k_c4_heavy_cost<<<grid_for(nh), kThreads, 0, s>>>(g->sym.row.p, g->dag.outdeg.p, heavy.p, hw.p,
                                                       nh, cost.p);
     GARY_CUDA(cudaGetLastError());
@@ -1188,25 +1237,37 @@ int launch_c4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaS
   // shards split the heavy tiles, the medium list and the light list
   auto part = [&](uint32_t total, uint32_t k) { return (uint32_t)((uint64_t)total * k / nshards); };
   const uint32_t t0 = part(plan->n_cta, shard), t1 = part(plan->n_cta, shard + 1);
-  const uint32_t m0 = part(plan->n_mid, shard), m1 = part(plan->n_mid, shard + 1);
+  const uint32_t n2 = plan->n_mid - plan->n_mid1;
+  const uint32_t m0 = part(plan->n_mid1, shard), m1 = part(plan->n_mid1, shard + 1);
+  const uint32_t q0 = plan->n_mid1 + part(n2, shard), q1 = plan->n_mid1 + part(n2, shard + 1);
   const uint32_t l0 = part(plan->n_light, shard), l1 = part(plan->n_light, shard + 1);
   const size_t smem_small = (size_t)kPWarps * 2 * kPSlots * 4;
-  const size_t smem_mid = (size_t)kMidWords * 4;
+  const size_t smem_mid = (size_t)mid_words(kMidLog) * 4, smem_mid1 = (size_t)mid_words(kMid1Log) * 4;
+  auto mid = k_c4_mid<kMidThreads, kMidLog, 2>;
+  auto mid1 = k_c4_mid<kMid1Threads, kMid1Log, 8>;
   const size_t smem_win = (size_t)kWinWords * 4;
   static bool attr[64] = {false};
   const int dev = device_ordinal();
   if (dev < 64 && !attr[dev]) {
     GARY_CUDA(cudaFuncSetAttribute(k_c4_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_small));
-    GARY_CUDA(cudaFuncSetAttribute(k_c4_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_mid));
+    GARY_CUDA(cudaFuncSetAttribute(mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_mid));
+    GARY_CUDA(cudaFuncSetAttribute(mid1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_mid1));
     attr[dev] = true;
   }
   GARY_TRY(c4_win_attr());
   int per_sm = 0;
   GARY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_c4_small, kPWarps * 32, smem_small));
   if (per_sm < 1) per_sm = 1;
-  int per_sm_mid = 0;
-  GARY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_mid, k_c4_mid, kMidThreads, smem_mid));
-  if (per_sm_mid < 1) per_sm_mid = 1;
+  auto grid = [&](auto kern, int threads, size_t smem, uint32_t items, unsigned &out) -> int {
+    int b = 0;
+    GARY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, threads, smem));
+    out = std::min<unsigned>((unsigned)(sm_count() * std::max(b, 1)), std::max(items, 1u));
+    return GARY_OK;
+  };
+  unsigned g_mid = 0, g_mid1 = 0;
+  GARY_TRY(grid(mid, kMidThreads, smem_mid, q1 - q0, g_mid));
+  GARY_TRY(grid(mid1, kMid1Threads, smem_mid1, m1 - m0, g_mid1));
+  SchedState *st = plan->sched.p;
   const GraphView sv{g->n, g->sym.row.p, g->sym.adj.p, true};
   GARY_CUDA(cudaMemsetAsync(plan->sched.p, 0, sizeof(SchedState), s));
   GARY_CUDA(cudaMemsetAsync(d_out, 0, 8, s));
@@ -1215,17 +1276,20 @@ int launch_c4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaS
   if (t1 > t0)
     k_c4_win<<<std::min<uint32_t>(plan->win_ctas, t1 - t0), kWinThreads, smem_win, s>>>(
         sv, plan->tiles.p, t0, t1, plan->cursors.p, std::max(plan->max_pre, 1u), plan->sched.p, d_out);
+  if (q1 > q0)
+    mid<<<g_mid, kMidThreads, smem_mid, s>>>(sv, g->dag.outdeg.p, plan->mid.p + q0, plan->mid_wed.p + q0, q1 - q0,
+                                             &st->next_aux, &st->error, d_out);
   if (m1 > m0)
-    k_c4_mid<<<std::min<uint32_t>((uint32_t)(sm_count() * per_sm_mid), m1 - m0), kMidThreads, smem_mid, s>>>(
-        sv, g->dag.outdeg.p, plan->mid.p + m0, m1 - m0, plan->sched.p, d_out);
+    mid1<<<g_mid1, kMid1Threads, smem_mid1, s>>>(sv, g->dag.outdeg.p, plan->mid.p + m0, plan->mid_wed.p + m0, m1 - m0,
+                                                 &st->next_mid1, &st->error, d_out);
   if (l1 > l0)
     k_c4_small<<<(unsigned)(sm_count() * per_sm), kPWarps * 32, smem_small, s>>>(
         sv, g->dag.outdeg.p, plan->light.p + l0, l1 - l0, plan->sched.p, d_out);
   GARY_CUDA(cudaGetLastError());
   GARY_CUDA(cudaEventRecord(g->ev1, s));
   g->last = gary_count_stats{};
-  g->last.tiles = (t1 - t0) + (m1 - m0) + (l1 - l0);
-  g->last.cta_tiles = (t1 - t0) + (m1 - m0);
+  g->last.tiles = (t1 - t0) + (q1 - q0) + (m1 - m0) + (l1 - l0);
+  g->last.cta_tiles = (t1 - t0) + (q1 - q0) + (m1 - m0);
   g->last_timed = true;
   g->last_sched = plan->sched.p;
   g->last_span = nullptr;

@@ -20,6 +20,10 @@ struct PatternPlan {
   DevBuf<uint32_t> cursors;  // C4: per window-kernel CTA, 6 x max_pre words of list state; K4: row pool
   AdjRows adj;               // K4: adjacency rows over the top ids
   C4Rows rows;               // C4: the vertices u counted by rows
+  // C4: medium vertices are mid[0 .. n_mid1) in the small map and the rest up to
+  // n_mid in the large one; mid_wed: their wedge counts
+  DevBuf<uint32_t> mid_wed;
+  uint32_t n_mid1 = 0;
   DevBuf<SchedState> sched;
   uint32_t n_cta = 0, n_warp = 0, n_light = 0, n_mid = 0, n_big = 0, n_pool = 0, max_pre = 0, win_ctas = 0;
 };

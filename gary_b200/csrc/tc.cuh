@@ -99,6 +99,7 @@ struct SchedState {
   uint32_t next_aux;  // a third queue (counted hub-row vertices; the 4-cycle kernel's medium vertices)
   uint32_t cta_path[4];  // triangle CTA tiles by the set that held N+(v) (kPath*)
   uint32_t next_big;     // a fourth queue (4-clique vertices whose rows fit shared memory)
+  uint32_t next_mid1;    // a fifth (the 4-cycle kernel's smaller medium vertices)
 };
 
 // Sets a triangle CTA tile can hold N+(v) in, cheapest first.
