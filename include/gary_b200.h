@@ -297,7 +297,8 @@ int gary_intersect_num_batch(uint64_t npairs, const uint64_t *d_a_off, const uin
 /* Search nkeys keys in one sorted list (duplicates allowed).  cache_entries = 0:
  * binary_search (include/ops/Search.cuh:48-61); otherwise the two-phase search
  * of Search.cuh:93-138 with that many samples cached per CTA (the reference
- * uses 32; up to 8192).  d_found[i] = 1 when keys[i] is present (optional);
+ * uses 32; up to 8192).  Batches of many keys take separators of the library's
+ * own number either way; the results do not depend on it.  d_found[i] = 1 when keys[i] is present (optional);
  * *d_count = number present (optional). */
 int gary_search_batch(const uint32_t *d_list, uint64_t len, const uint32_t *d_keys, uint64_t nkeys,
                       uint32_t cache_entries, uint8_t *d_found, uint64_t *d_count, void *stream);

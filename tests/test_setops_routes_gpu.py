@@ -91,3 +91,20 @@ def test_bounds_and_exclusions(pairs, variant):
     counts, total = so.intersect_num(batch, t(bound, np.int32), t(np.array(off, np.int64), np.int64),
                                      t(np.array(ex, np.uint32), np.int32), so.VARIANTS[variant])
     assert counts.cpu().tolist() == want and int(total.item()) == sum(want)
+
+
+@pytest.mark.parametrize("n_list", [8191, 8192, 8193, 16385, 65543, (1 << 20) + 13])
+@pytest.mark.parametrize("n_keys", [606207, 606208, 1300007, 5000003])
+def test_search_of_many_keys(cuda, n_list, n_keys):
+    """Every depth of the separator tree, lists with repeated ids and the ids at
+    both ends of the range."""
+    import torch
+
+    rng = np.random.default_rng(n_list + n_keys)
+    lst = np.sort(rng.integers(0, 4 * n_list, n_list).astype(np.uint32))
+    lst[0], lst[-1], lst[-2] = 0, 0xFFFFFFFE, 0xFFFFFFFE
+    keys = rng.integers(0, 4 * n_list + 8, n_keys).astype(np.uint32)
+    keys[:4] = [0, 0xFFFFFFFE, 0xFFFFFFFF, 0xFFFFFFFD]
+    found, count = so.search(torch.from_numpy(lst.view(np.int32)).cuda(), torch.from_numpy(keys.view(np.int32)).cuda(), 256)
+    want = np.isin(keys, lst)
+    assert np.array_equal(found.cpu().numpy().astype(bool), want) and int(count.item()) == int(want.sum())
