@@ -67,55 +67,74 @@ struct MinU64 {
   __host__ __device__ uint64_t operator()(uint64_t a, uint64_t b) const { return a < b ? a : b; }
 };
 
-// One candidate per padded word w of N+(u): the suffix after v = adj[w], up to
-// len[u] (null: the whole list); *cut += the suffix ids past len[u].
-// Words without a record get the key n - 1: in rank ids the top vertex has
-// no higher neighbour, so no record ever targets it, and the keys of an
-// n = 2^k graph fit k bits (one radix pass fewer than with the key n).
-__global__ void k_in_candidates(const uint2 *__restrict__ row, const uint32_t *__restrict__ adj,
-                                const uint32_t *__restrict__ rowid, uint64_t words, uint32_t n,
-                                const uint32_t *__restrict__ len, uint32_t *__restrict__ keys,
-                                uint2 *__restrict__ vals, unsigned long long *__restrict__ cut) {
+// The records of the padded words w of N+(u): the suffix after v = adj[w], up to
+// len[u] (null: the whole list), keyed by v.  Records are appended tile by tile
+// (in word order within a tile of kCandTile words, one atomic a tile), so the
+// sort that follows moves records only: after hub rows have taken the hub
+// suffixes a third of the words hold one at RMAT-20 ef16.  *cut += the suffix
+// ids past len[u]; *count: the records.
+constexpr int kCandPer = 8;
+constexpr uint32_t kCandTile = kThreads * kCandPer;
+__global__ void __launch_bounds__(kThreads)
+    k_in_candidates(const uint2 *__restrict__ row, const uint32_t *__restrict__ adj,
+                    const uint32_t *__restrict__ rowid, uint64_t words, const uint32_t *__restrict__ len,
+                    uint32_t *__restrict__ keys, uint2 *__restrict__ vals, unsigned long long *__restrict__ cut,
+                    unsigned long long *__restrict__ count) {
+  constexpr int kW = kThreads / 32;
+  __shared__ uint32_t at[kCandPer * kW];
+  __shared__ unsigned long long s_base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long mine = 0;
-  for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < words;
-       w += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t u = rowid[w];
-    const uint2 r = row[u];
-    const uint64_t pos = w - (uint64_t)r.x * 4;
-    uint32_t key = n - 1;
-    uint2 val = make_uint2(0, 0);
-    if (pos < r.y) {
-      const uint32_t v = adj[w];
-      const uint32_t rem = r.y - (uint32_t)pos - 1;
-      if (rem && row[v].y) {
-        const uint32_t end = len ? len[u] : r.y;
-        const uint32_t keep = end > (uint32_t)pos + 1 ? end - (uint32_t)pos - 1 : 0u;
-        mine += rem - keep;
-        if (keep) {
-          key = v;
-          val = make_uint2((uint32_t)(w + 1), keep);
+  for (uint64_t t0 = (uint64_t)blockIdx.x * kCandTile; t0 < words; t0 += (uint64_t)gridDim.x * kCandTile) {
+    uint32_t key[kCandPer];
+    uint32_t keep[kCandPer];
+    unsigned has[kCandPer];
+#pragma unroll
+    for (int i = 0; i < kCandPer; ++i) {
+      const uint64_t w = t0 + (uint64_t)i * kThreads + threadIdx.x;
+      key[i] = 0;
+      keep[i] = 0;
+      if (w < words) {
+        const uint32_t u = rowid[w];
+        const uint2 r = row[u];
+        const uint64_t pos = w - (uint64_t)r.x * 4;
+        if (pos < r.y) {
+          const uint32_t v = adj[w];
+          const uint32_t rem = r.y - (uint32_t)pos - 1;
+          if (rem && row[v].y) {
+            const uint32_t end = len ? len[u] : r.y;
+            keep[i] = end > (uint32_t)pos + 1 ? end - (uint32_t)pos - 1 : 0u;
+            mine += rem - keep[i];
+            key[i] = v;
+          }
         }
       }
+      has[i] = __ballot_sync(kFull, keep[i] != 0);
+      if (lane == 0) at[i * kW + warp] = __popc(has[i]);
     }
-    keys[w] = key;
-    vals[w] = val;
+    __syncthreads();
+    if (warp == 0) {  // where each warp's part of each row of the tile goes
+      uint32_t a = at[2 * lane], b = at[2 * lane + 1];
+      const uint32_t incl = warp_inclusive_sum(a + b, lane);
+      if (lane == 31) s_base = atomicAdd(count, (unsigned long long)incl);
+      at[2 * lane] = incl - a - b;
+      at[2 * lane + 1] = incl - b;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kCandPer; ++i)
+      if (keep[i]) {
+        const uint64_t o = s_base + at[i * kW + warp] + __popc(has[i] & ((1u << lane) - 1u));
+        keys[o] = key[i];
+        vals[o] = make_uint2((uint32_t)(t0 + (uint64_t)i * kThreads + threadIdx.x + 1), keep[i]);
+      }
+    __syncthreads();
   }
+  static_assert(kCandPer * kW == 64, "two entries a lane");
   if (len) {
     mine = warp_sum_u64(mine);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(cut, mine);
+    if (lane == 0 && mine) atomicAdd(cut, mine);
   }
-}
-
-// first index i with keys[i] >= x in a sorted array (one thread)
-__global__ void k_first_geq(const uint32_t *__restrict__ keys, uint64_t len, uint32_t x,
-                            uint64_t *__restrict__ out) {
-  uint64_t b = 0, e = len;
-  while (b < e) {
-    const uint64_t m = (b + e) >> 1;
-    if (keys[m] < x) b = m + 1;
-    else e = m;
-  }
-  *out = b;
 }
 
 __global__ void k_in_heads(const uint32_t *__restrict__ keys, uint64_t m,
@@ -333,45 +352,41 @@ int build_in_index(gary_graph *g, cudaStream_t s, const DevBuf<uint32_t> &len, I
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
   DevBuf<uint32_t> keys, keys2;
   DevBuf<uint2> vals, vals2;
-  DevBuf<unsigned long long> cut;
-  GARY_TRY(cut.alloc(1, s));
+  uint64_t m = 0;
   {
     DevBuf<uint32_t> rowid;
+    DevBuf<unsigned long long> cut;  // {suffix ids cut off, records}
+    GARY_TRY(cut.alloc(2, s));
+    GARY_CUDA(cudaMemsetAsync(cut.p, 0, 16, s));
     GARY_TRY(padded_rowid(g->dag, rowid, s));
-    GARY_TRY(keys.alloc(W, s));
-    GARY_TRY(vals.alloc(W, s));
-    GARY_CUDA(cudaMemsetAsync(cut.p, 0, 8, s));
-    k_in_candidates<<<grid_for(W), kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, n, len.p, keys.p,
-                                                     vals.p, cut.p);
+    GARY_TRY(keys.alloc(std::max<uint64_t>(W, 1), s));
+    GARY_TRY(vals.alloc(std::max<uint64_t>(W, 1), s));
+    if (W)
+      k_in_candidates<<<grid_for((W + kCandPer - 1) / kCandPer), kThreads, 0, s>>>(
+          g->dag.row.p, g->dag.adj.p, rowid.p, W, len.p, keys.p, vals.p, cut.p, cut.p + 1);
     GARY_CUDA(cudaGetLastError());
+    unsigned long long h[2] = {0, 0};
+    GARY_CUDA(cudaMemcpyAsync(h, cut.p, 16, cudaMemcpyDeviceToHost, s));
+    GARY_CUDA(cudaStreamSynchronize(s));
+    in.hub_work = h[0];
+    m = h[1];
   }
-  GARY_TRY(keys2.alloc(W, s));
-  GARY_TRY(vals2.alloc(W, s));
-  {
+  if (m) {
+    GARY_TRY(keys2.alloc(m, s));
+    GARY_TRY(vals2.alloc(m, s));
     cub::DoubleBuffer<uint32_t> kb(keys.p, keys2.p);
     cub::DoubleBuffer<uint2> vb(vals.p, vals2.p);
     size_t tmp = 0;
-    const int eb = bits_for((uint64_t)n);  // keys <= n - 1
-    GARY_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, kb, vb, W, 0, eb, s));
+    const int eb = bits_for((uint64_t)n);
+    GARY_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, kb, vb, m, 0, eb, s));
     DevBuf<uint8_t> t;
     GARY_TRY(t.alloc(tmp, s));
-    GARY_CUDA(cub::DeviceRadixSort::SortPairs(t.p, tmp, kb, vb, W, 0, eb, s));
+    GARY_CUDA(cub::DeviceRadixSort::SortPairs(t.p, tmp, kb, vb, m, 0, eb, s));
     if (kb.Current() != keys.p) std::swap(keys, keys2);
     if (vb.Current() != vals.p) std::swap(vals, vals2);
   }
   keys2.release();
   vals2.release();
-  // records = number of keys < n - 1 (the rest carry the "no record" key n - 1)
-  uint64_t m = 0;
-  {
-    DevBuf<uint64_t> pos;
-    GARY_TRY(pos.alloc(1, s));
-    k_first_geq<<<1, 1, 0, s>>>(keys.p, W, n - 1, pos.p);
-    GARY_CUDA(cudaGetLastError());
-    GARY_CUDA(cudaMemcpyAsync(&m, pos.p, 8, cudaMemcpyDeviceToHost, s));
-    GARY_CUDA(cudaMemcpyAsync(&in.hub_work, cut.p, 8, cudaMemcpyDeviceToHost, s));
-    GARY_CUDA(cudaStreamSynchronize(s));
-  }
   in.records = m;
   GARY_TRY(in.inptr.alloc_persistent((uint64_t)n + 1));
   thrust::fill(pol, in.inptr.p, in.inptr.p + n + 1, m);
