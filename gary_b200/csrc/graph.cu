@@ -557,9 +557,8 @@ int radix_sort_keys(DevBuf<uint64_t> &keys, DevBuf<uint64_t> &alt, uint64_t m, i
 }
 
 int row_starts(const DevBuf<uint64_t> &keys, uint64_t m, uint32_t n, int lg,
-               DevBuf<uint64_t> &rowstart, cudaStream_t s, bool persistent = false) {
-  if (persistent) GARY_TRY(rowstart.alloc_persistent((uint64_t)n + 1));
-  else GARY_TRY(rowstart.alloc((uint64_t)n + 1, s));
+               DevBuf<uint64_t> &rowstart, cudaStream_t s) {
+  GARY_TRY(rowstart.alloc((uint64_t)n + 1, s));
   // fill with m, heads, then reverse min-scan so empty rows point at the next row
   ScratchAlloc pol_alloc{s};
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
@@ -607,23 +606,6 @@ int compact_keys(DevBuf<uint64_t> &keys, uint64_t count, uint64_t &kept, cudaStr
   DevBuf<uint8_t> t;
   GARY_TRY(t.alloc(tmp, s));
   GARY_CUDA(cub::DeviceSelect::If(t.p, tmp, keys.p, out.p, nsel.p, (int64_t)count, NotAllOnes(), s));
-  GARY_CUDA(cudaMemcpyAsync(&kept, nsel.p, 8, cudaMemcpyDeviceToHost, s));
-  GARY_CUDA(cudaStreamSynchronize(s));
-  std::swap(keys, out);
-  return GARY_OK;
-}
-
-int unique_keys(DevBuf<uint64_t> &keys, uint64_t count, uint64_t &kept, cudaStream_t s) {
-  kept = 0;
-  if (!count) return GARY_OK;
-  DevBuf<uint64_t> out, nsel;
-  GARY_TRY(out.alloc(count, s));
-  GARY_TRY(nsel.alloc(1, s));
-  size_t tmp = 0;
-  GARY_CUDA(cub::DeviceSelect::Unique(nullptr, tmp, keys.p, out.p, nsel.p, (int64_t)count, s));
-  DevBuf<uint8_t> t;
-  GARY_TRY(t.alloc(tmp, s));
-  GARY_CUDA(cub::DeviceSelect::Unique(t.p, tmp, keys.p, out.p, nsel.p, (int64_t)count, s));
   GARY_CUDA(cudaMemcpyAsync(&kept, nsel.p, 8, cudaMemcpyDeviceToHost, s));
   GARY_CUDA(cudaStreamSynchronize(s));
   std::swap(keys, out);
@@ -1060,30 +1042,152 @@ int upload(const uint64_t *ptr, const uint32_t *idx, uint32_t n, uint64_t nnz, u
 
 // ---------------------------------------------------------------------------
 // Symmetric CSR from an undirected edge list (dedup, drop loops, symmetrise).
+//
+// Every edge is sorted once, as (smaller end, larger end), not in both
+// directions: the sort is the cost (98 G 8-byte keys/s a pass of 8 bits), and
+// half the keys make half of it.  Loops are dropped with the duplicates, as keys
+// whose two ends are equal, so no pass compacts the keys first.  The sorted
+// distinct edges are the larger-neighbour lists; stably sorted by their larger
+// end they are the smaller-neighbour lists, each in order, and a row of the CSR
+// is the one after the other.
 namespace {
 __global__ void k_edge_keys(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst,
                             uint64_t m, uint32_t n, int lg, uint64_t *__restrict__ keys,
                             unsigned *err) {
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
        i += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t a = src[i], b = dst[i];
+    const uint32_t a = src[i], b = dst[i];
     if (a >= n || b >= n) {
       atomicOr(err, kErrRange);
-      keys[2 * i] = keys[2 * i + 1] = ~0ull;
-    } else if (a == b) {
-      keys[2 * i] = keys[2 * i + 1] = ~0ull;
+      keys[i] = 0;
     } else {
-      keys[2 * i] = ((uint64_t)a << lg) | b;
-      keys[2 * i + 1] = ((uint64_t)b << lg) | a;
+      keys[i] = ((uint64_t)min(a, b) << lg) | max(a, b);
     }
   }
 }
-__global__ void k_key_cols(const uint64_t *__restrict__ keys, uint64_t m, int lg,
-                           uint32_t *__restrict__ idx) {
+
+// An edge of the sorted keys is kept when it is no loop and the first of its kind.
+__device__ __forceinline__ bool first_of_edge(const uint64_t *__restrict__ keys, uint64_t i, int lg, uint64_t &key) {
+  key = keys[i];
+  return (i == 0 || keys[i - 1] != key) && (key >> lg) != (key & ((1ull << lg) - 1));
+}
+
+// Kept keys per tile of kEdgeTile.
+constexpr int kEdgePer = 16;
+constexpr uint32_t kEdgeTile = kThreads * kEdgePer;
+__global__ void __launch_bounds__(kThreads)
+    k_edge_count(const uint64_t *__restrict__ keys, uint64_t m, int lg, uint64_t *__restrict__ tiles) {
+  __shared__ uint32_t s_n;
+  for (uint64_t t = blockIdx.x; t * kEdgeTile < m; t += gridDim.x) {
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    uint32_t c = 0;
+    for (int i = 0; i < kEdgePer; ++i) {
+      const uint64_t at = t * kEdgeTile + (uint64_t)i * kThreads + threadIdx.x;
+      uint64_t key;
+      c += at < m && first_of_edge(keys, at, lg, key);
+    }
+    c = __reduce_add_sync(kFull, c);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&s_n, c);
+    __syncthreads();
+    if (threadIdx.x == 0) tiles[t] = s_n;
+    __syncthreads();
+  }
+}
+
+// Up to so many tiles, each adds up the counts before it itself: a scan's two
+// launches cost a small graph more than the sort.
+constexpr uint64_t kEdgeFewTiles = 128;
+
+// The kept edges, their ends apart.  tiles: each tile's offset (scanned) or its
+// count.
+__global__ void __launch_bounds__(kThreads)
+    k_edge_write(const uint64_t *__restrict__ keys, uint64_t m, int lg, const uint64_t *__restrict__ tiles,
+                 bool scanned, uint32_t *__restrict__ lo, uint32_t *__restrict__ hi) {
+  constexpr int kW = kThreads / 32;
+  __shared__ uint32_t at[kEdgePer * kW];
+  __shared__ uint64_t s_base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t mask = (1ull << lg) - 1;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    idx[i] = (uint32_t)(keys[i] & mask);
+  for (uint64_t t = blockIdx.x; t * kEdgeTile < m; t += gridDim.x) {
+    uint64_t key[kEdgePer];
+    unsigned has[kEdgePer];
+#pragma unroll
+    for (int i = 0; i < kEdgePer; ++i) {
+      const uint64_t w = t * kEdgeTile + (uint64_t)i * kThreads + threadIdx.x;
+      key[i] = 0;
+      const bool k = w < m && first_of_edge(keys, w, lg, key[i]);
+      has[i] = __ballot_sync(kFull, k);
+      if (lane == 0) at[i * kW + warp] = __popc(has[i]);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t c[4], sum = 0;
+      for (int j = 0; j < 4; ++j) sum += c[j] = at[4 * lane + j];
+      uint32_t incl = sum;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (scanned) {
+        if (lane == 0) s_base = tiles[t];
+      } else {
+        uint32_t before = 0;  // at most 128 tiles of 4096
+        for (uint64_t j = lane; j < t; j += 32) before += (uint32_t)tiles[j];
+        before = __reduce_add_sync(kFull, before);
+        if (lane == 0) s_base = before;
+      }
+      uint32_t x = incl - sum;
+      for (int j = 0; j < 4; ++j) {
+        at[4 * lane + j] = x;
+        x += c[j];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kEdgePer; ++i)
+      if ((has[i] >> lane) & 1u) {
+        const uint64_t o = s_base + at[i * kW + warp] + __popc(has[i] & ((1u << lane) - 1u));
+        lo[o] = (uint32_t)(key[i] >> lg);
+        hi[o] = (uint32_t)(key[i] & mask);
+      }
+    __syncthreads();
+  }
+  static_assert(kEdgePer * kW == 128, "four entries a lane");
+}
+
+// Where u's edges begin among the sorted smaller ends (up) and larger ends
+// (down), and so its row, for u = 0 .. n.  Two binary searches a vertex, in one
+// launch: marking the heads and scanning over the gaps takes seven.
+__global__ void k_end_starts(const uint32_t *__restrict__ lo, const uint32_t *__restrict__ dhi, uint64_t k, uint32_t n,
+                             uint64_t *__restrict__ up, uint64_t *__restrict__ down, uint64_t *__restrict__ ptr) {
+  auto first = [&](const uint32_t *ends, uint64_t u) {
+    uint64_t b = 0, e = k;
+    while (b < e) {
+      const uint64_t m = (b + e) >> 1;
+      if (ends[m] < u) b = m + 1;
+      else e = m;
+    }
+    return b;
+  };
+  for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u <= n; u += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t a = first(lo, u), b = first(dhi, u);
+    up[u] = a;
+    down[u] = b;
+    ptr[u] = a + b;
+  }
+}
+
+// Row u: its smaller neighbours (down, the lists by larger end) and then its
+// larger ones (up).  An edge's place follows from the other direction's starts.
+__global__ void k_csr_rows(const uint32_t *__restrict__ lo, const uint32_t *__restrict__ hi,
+                           const uint32_t *__restrict__ dhi, const uint32_t *__restrict__ dlo, uint64_t k,
+                           const uint64_t *__restrict__ up, const uint64_t *__restrict__ down,
+                           uint32_t *__restrict__ idx) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < k; i += (uint64_t)gridDim.x * blockDim.x) {
+    idx[i + down[(uint64_t)lo[i] + 1]] = hi[i];
+    idx[i + up[dhi[i]]] = dlo[i];
+  }
 }
 }  // namespace
 
@@ -1111,31 +1215,63 @@ int csr_from_edges(const uint32_t *src, const uint32_t *dst, uint64_t m, uint32_
   DevBuf<unsigned> err;
   GARY_TRY(err.alloc(1, s));
   GARY_CUDA(cudaMemsetAsync(err.p, 0, 4, s));
-  DevBuf<uint64_t> keys, alt;
-  uint64_t k = 0;
-  GARY_TRY(keys.alloc(std::max<uint64_t>(2 * m, 1), s));
-  if (m) {
-    k_edge_keys<<<grid_for(m), kThreads, 0, s>>>(src, dst, m, n, lg, keys.p, err.p);
+  uint64_t k = 0;  // distinct edges
+  DevBuf<uint32_t> lo, hi;
+  {
+    DevBuf<uint64_t> keys, alt;
+    GARY_TRY(keys.alloc(std::max<uint64_t>(m, 1), s));
+    GARY_TRY(alt.alloc(std::max<uint64_t>(m, 1), s));
+    if (m) k_edge_keys<<<grid_for(m), kThreads, 0, s>>>(src, dst, m, n, lg, keys.p, err.p);
     GARY_CUDA(cudaGetLastError());
-    GARY_TRY(compact_keys(keys, 2 * m, k, s));
+    s_own.release();
+    d_own.release();
+    if (m) GARY_TRY(radix_sort_keys(keys, alt, m, 2 * lg, s));
+    alt.release();
+    const uint64_t nt = (m + kEdgeTile - 1) / kEdgeTile;
+    DevBuf<uint64_t> tiles;
+    GARY_TRY(tiles.alloc(nt + 1, s));
+    const unsigned tile_grid = grid_for(nt * kThreads);
+    const bool scan = nt > kEdgeFewTiles;
+    if (m) k_edge_count<<<tile_grid, kThreads, 0, s>>>(keys.p, m, lg, tiles.p);
+    GARY_CUDA(cudaGetLastError());
+    uint64_t few[kEdgeFewTiles] = {0};
+    if (scan) {
+      GARY_CUDA(cudaMemsetAsync(tiles.p + nt, 0, 8, s));
+      thrust::exclusive_scan(pol, tiles.p, tiles.p + nt + 1, tiles.p, 0ull);
+      GARY_CUDA(cudaMemcpyAsync(&k, tiles.p + nt, 8, cudaMemcpyDeviceToHost, s));
+    } else if (nt) {
+      GARY_CUDA(cudaMemcpyAsync(few, tiles.p, nt * 8, cudaMemcpyDeviceToHost, s));
+    }
+    unsigned herr = 0;
+    GARY_TRY(read_err(err.p, s, &herr));
+    if (herr) return input_error(herr);
+    for (uint64_t t = 0; !scan && t < nt; ++t) k += few[t];
+    GARY_TRY(lo.alloc(std::max<uint64_t>(k, 1), s));
+    GARY_TRY(hi.alloc(std::max<uint64_t>(k, 1), s));
+    if (k) k_edge_write<<<tile_grid, kThreads, 0, s>>>(keys.p, m, lg, tiles.p, scan, lo.p, hi.p);
+    GARY_CUDA(cudaGetLastError());
   }
-  s_own.release();
-  d_own.release();
-  unsigned herr = 0;
-  GARY_TRY(read_err(err.p, s, &herr));
-  if (herr) return input_error(herr);
-  GARY_TRY(alt.alloc(std::max<uint64_t>(k, 1), s));
+  // the same edges by larger end, the smaller ends in order
+  DevBuf<uint32_t> dhi, dlo;
+  GARY_TRY(dhi.alloc(std::max<uint64_t>(k, 1), s));
+  GARY_TRY(dlo.alloc(std::max<uint64_t>(k, 1), s));
   if (k) {
-    GARY_TRY(radix_sort_keys(keys, alt, k, 2 * lg, s));
-    GARY_TRY(unique_keys(keys, k, k, s));
+    size_t tmp = 0;
+    GARY_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, hi.p, dhi.p, lo.p, dlo.p, k, 0, lg, s));
+    DevBuf<uint8_t> t;
+    GARY_TRY(t.alloc(tmp, s));
+    GARY_CUDA(cub::DeviceRadixSort::SortPairs(t.p, tmp, hi.p, dhi.p, lo.p, dlo.p, k, 0, lg, s));
   }
-  alt.release();
-  DevBuf<uint64_t> rowstart;
-  GARY_TRY(row_starts(keys, k, n, lg, rowstart, s, true));
-  GARY_TRY(c->idx.alloc_persistent(std::max<uint64_t>(k, 1)));
-  if (k) k_key_cols<<<grid_for(k), kThreads, 0, s>>>(keys.p, k, lg, c->idx.p);
+  DevBuf<uint64_t> starts;
+  GARY_TRY(starts.alloc(2 * ((uint64_t)n + 1), s));
+  uint64_t *up = starts.p, *down = up + n + 1;
+  GARY_TRY(c->ptr.alloc_persistent((uint64_t)n + 1));
+  GARY_TRY(c->idx.alloc_persistent(std::max<uint64_t>(2 * k, 1)));
+  k_end_starts<<<grid_for((uint64_t)n + 1), kThreads, 0, s>>>(lo.p, dhi.p, k, n, up, down, c->ptr.p);
+  if (k)
+    k_csr_rows<<<grid_for(k), kThreads, 0, s>>>(lo.p, hi.p, dhi.p, dlo.p, k, up, down, c->idx.p);
   GARY_CUDA(cudaGetLastError());
-  c->ptr = std::move(rowstart);
+  k *= 2;
   c->nnz = k;
   GARY_CUDA(cudaStreamSynchronize(s));
   *out = c.release();
