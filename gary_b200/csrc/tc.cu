@@ -768,23 +768,23 @@ __device__ __forceinline__ void add_graph_count(const VertexCtl &ctl, uint32_t v
   if (lane == 0 && t) atomicAdd(&ctl.gcount[ctl.gid[v]], t);
 }
 
-// One middle vertex v on one warp: a set of N+(v) in the warp's slots, walk
-// in-edges [j0, j1) of v.
-__device__ __forceinline__ uint32_t warp_vertex(const GraphView &g, const uint2 *__restrict__ inedge,
-                                                const uint64_t *__restrict__ inptr, uint32_t v,
-                                                uint32_t j0, uint32_t j1, uint32_t *tab, int lane,
-                                                const VertexCtl &ctl) {
-  const uint2 rv = g.row[v];
-  const uint32_t d = rv.y;
-  const uint64_t base = inptr[v];
-  const uint64_t nin = inptr[v + 1] - base;
-  const uint64_t ke = base + min_u64(j1, nin);
-  const uint64_t kb = base + j0;
-  if (d == 0 || kb >= ke) return 0;
+// What a warp needs of a middle vertex before it builds a set: its list, its
+// records [kb, ke) and the list's first id and span.
+struct VertexHead {
+  uint2 rv;
+  uint32_t lo, span;
+  uint64_t kb, ke;
+};
+
+// One middle vertex v (d+ > 0, some records) on one warp: a set of N+(v) in the
+// warp's slots, walk its records.
+__device__ __forceinline__ uint32_t warp_vertex(const GraphView &g, const uint2 *__restrict__ inedge, uint32_t v,
+                                                const VertexHead &h, uint32_t *tab, int lane, const VertexCtl &ctl) {
+  const uint32_t d = h.rv.y, lo = h.lo, span = h.span;
+  const uint64_t kb = h.kb, ke = h.ke;
   const long long t0 = ctl.cycles ? clock64() : 0;
-  const uint32_t *av = g.adj + (uint64_t)rv.x * 4;
+  const uint32_t *av = g.adj + (uint64_t)h.rv.x * 4;
   const uint4 *adj4 = reinterpret_cast<const uint4 *>(g.adj);
-  const uint32_t lo = av[0], span = av[d - 1] - lo;
   auto sync = [] { __syncwarp(); };
   uint32_t var = span <= kWarpBitmapSpan ? kVarBitmap : kVarHash;
   if (ctl.variant) {
@@ -830,26 +830,24 @@ __device__ __forceinline__ uint32_t match_octets(const uint4 &a, const uint4 &b,
   return in(a.x) + in(a.y) + in(a.z) + in(a.w) + in(b.x) + in(b.y) + in(b.z) + in(b.w);
 }
 
-// All in-edges of the tiny vertices among 32 light ones (lane's v, where
-// `tiny`), without a set: the 32 vertices' records are walked flattened, and
+// All in-edges of the tiny vertices among 32 light ones (lane's list rv and its
+// nin_v records from ib on, where `tiny`), without a set: the 32 vertices' records are walked flattened, and
 // within a batch of 32 records their octets are, so every lane compares one
 // octet of a suffix with the one or two octets of N+(v).  Building a set costs
 // a vertex some thousands of cycles of dependent loads and shared-memory
 // passes whatever its size, which for these vertices is most of their time.
 // All 32 lanes must call.
-__device__ __forceinline__ uint32_t tiny_vertices(const GraphView &g, const uint2 *__restrict__ inedge,
-                                                  const uint64_t *__restrict__ inptr, uint32_t v, uint2 rv,
-                                                  bool tiny, int lane) {
+__device__ __forceinline__ uint32_t tiny_vertices(const GraphView &g, const uint2 *__restrict__ inedge, uint32_t ib,
+                                                  uint32_t nin_v, uint2 rv, bool tiny, int lane) {
   // N+(v)'s padding equals a suffix's padding: the suffix's is lowered by one
   // (still no vertex id), which is also what lanes without an octet hold.
   constexpr uint32_t kNever = kSentinel - 1u;
   const uint4 *adj4 = reinterpret_cast<const uint4 *>(g.adj);
-  const uint64_t ib = tiny ? inptr[v] : 0;
-  const uint32_t nin = tiny ? (uint32_t)(inptr[v + 1] - ib) : 0u;
+  const uint32_t nin = tiny ? nin_v : 0u;
   const uint32_t incl = warp_inclusive_sum(nin, lane);
   const uint32_t records = __shfl_sync(kFull, incl, 31);
   // record of flattened position p: rbias + p (mod 2^32, as the octets below) of the owner
-  const uint32_t rbias = (uint32_t)ib - (incl - nin);
+  const uint32_t rbias = ib - (incl - nin);
   const uint32_t myset = (rv.x >> 1) | (rv.y > 8 ? 1u << 31 : 0u);  // N+(v)'s first octet; bit 31: it has two
   WarpRuns runs(incl - nin, nin, lane);
   uint32_t cnt = 0;
@@ -963,8 +961,12 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
       t = __shfl_sync(kFull, t, 0);
       if (t >= rng.warp_hi) break;
       const Tile tl = wt[t];
-      if (tl.j1 != kGroupTile) {
-        cnt += warp_vertex(g, inedge, inptr, tl.v0, tl.j0, tl.j1, tab, lane, ctl);
+      if (tl.j1 != kGroupTile) {  // records [j0, j1) of one vertex
+        const uint2 rv = g.row[tl.v0];
+        const uint32_t *av = g.adj + (uint64_t)rv.x * 4;
+        const uint64_t base = inptr[tl.v0];
+        const uint32_t lo = av[0];
+        cnt += warp_vertex(g, inedge, tl.v0, VertexHead{rv, lo, av[rv.y - 1] - lo, base + tl.j0, base + tl.j1}, tab, lane, ctl);
         continue;
       }
       // a group of light vertices: list positions [v0, v1), 32 ids per load
@@ -981,12 +983,21 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
           together = __all_sync(kFull, lane >= nb || gid == g0);
           gid = g0;
         }
+        // the heads of all 32 in lanes, so that the loads a vertex begins with
+        // are waited for once, not by every vertex again
+        uint2 rv = make_uint2(0, 0);
+        uint64_t kb = 0;
+        uint32_t nin = 0;
+        if (lane < nb) {
+          rv = g.row[myv];
+          kb = inptr[myv];
+          nin = (uint32_t)(inptr[myv + 1] - kb);
+        }
         if (together) {
-          const uint2 rv = lane < nb ? g.row[myv] : make_uint2(0, 0);
           const bool tiny = rv.y - 1u < kTinyOut;
           const unsigned tm = __ballot_sync(kFull, tiny);
           if (tm) {
-            const uint32_t c = tiny_vertices(g, inedge, inptr, myv, rv, tiny, lane);
+            const uint32_t c = tiny_vertices(g, inedge, (uint32_t)kb, nin, rv, tiny, lane);
             cnt += c;
             if (ctl.gcount) {
               const unsigned long long sum = warp_sum_u64(c);
@@ -995,10 +1006,25 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
             left &= ~tm;
           }
         }
-        while (left) {
-          const int k = __ffs(left) - 1;
-          left &= left - 1;
-          cnt += warp_vertex(g, inedge, inptr, __shfl_sync(kFull, myv, k), 0, 0xFFFFFFFFu, tab, lane, ctl);
+        if (left) {
+          uint32_t lo = 0, span = 0;
+          if ((left >> lane) & 1u) {
+            const uint32_t *av = g.adj + (uint64_t)rv.x * 4;
+            lo = av[0];
+            span = av[rv.y - 1] - lo;
+          }
+          while (left) {
+            const int k = __ffs(left) - 1;
+            left &= left - 1;
+            VertexHead h;
+            h.rv.x = __shfl_sync(kFull, rv.x, k);
+            h.rv.y = __shfl_sync(kFull, rv.y, k);
+            h.lo = __shfl_sync(kFull, lo, k);
+            h.span = __shfl_sync(kFull, span, k);
+            h.kb = __shfl_sync(kFull, (uint32_t)kb, k);  // records are numbered in 32 bits (build_in_index)
+            h.ke = h.kb + __shfl_sync(kFull, nin, k);
+            cnt += warp_vertex(g, inedge, __shfl_sync(kFull, myv, k), h, tab, lane, ctl);
+          }
         }
       }
     }
