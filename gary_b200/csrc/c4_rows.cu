@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "c4_rows.cuh"
+#include "hub.cuh"
 #include "warp_ops.cuh"
 
 namespace gary {
@@ -335,7 +336,9 @@ struct DegreeIn {
 
 }  // namespace
 
-int build_c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
+namespace {
+
+int c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
   const uint32_t n = g->n;
   const uint2 *row = g->sym.row.p;
   const uint32_t *adj = g->sym.adj.p, *dplus = g->dag.outdeg.p;
@@ -354,9 +357,7 @@ int build_c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
   unsigned long long h[kC4MaxSlabs + 1];
   GARY_CUDA(cudaMemcpyAsync(h, stat.p, sizeof(h), cudaMemcpyDeviceToHost, s));
   GARY_CUDA(cudaStreamSynchronize(s));
-  size_t free_bytes = 0, total_bytes = 0;
-  GARY_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
-  uint64_t room = total_bytes / 8;  // for all slabs' rows
+  uint64_t used = 0;  // by all slabs' rows
   DevBuf<uint32_t> list;
   GARY_TRY(list.alloc(n, s));
   for (int k = 0; k < se.slabs && h[k] && h[k] / kC4RowWedges >= h[kC4MaxSlabs]; ++k) {
@@ -368,8 +369,8 @@ int build_c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
                                                    thrust::counting_iterator<uint32_t>(n), list.p,
                                                    TouchesSlab{row, adj, sl.first, sl.end}) - list.p);
     const uint64_t bytes = ((uint64_t)span + nl + 1) * kC4RowQuads * 16;
-    if (bytes > room) break;
-    room -= bytes;
+    if (!room_for_rows(used + bytes)) break;
+    used += bytes;
     GARY_TRY(sl.rowof.alloc_persistent(n));
     GARY_TRY(sl.rows.alloc_persistent(bytes / 16));
     sl.zero = span + nl;
@@ -390,6 +391,19 @@ int build_c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
   r.n5 = pick(r.list.p, 2, 31);
   r.n8 = pick(r.list.p + r.n5, 32, 255);
   r.n32 = pick(r.list.p + r.n5 + r.n8, 256, 0xFFFFFFFFu);
+  return GARY_OK;
+}
+
+}  // namespace
+
+int build_c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
+  const int rc = c4_rows(g, s, r);
+  if (rc != GARY_ERR_OOM) return rc;
+  // no room on the device: the wedge kernels take every vertex
+  GARY_CUDA(cudaStreamSynchronize(s));
+  r = C4Rows{};
+  r.lowest = g->n;
+  clear_error();
   return GARY_OK;
 }
 

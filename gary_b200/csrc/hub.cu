@@ -158,7 +158,9 @@ __global__ void k_adj_low(const uint2 *__restrict__ row, const uint32_t *__restr
 
 }  // namespace
 
-int build_adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj) {
+namespace {
+
+int adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj) {
   const uint32_t n = g->n, span = std::min(n, kAdjRowIds), first = n - span;
   adj.words = 0;
   if (g->dag.max_len < 3) return GARY_OK;
@@ -181,9 +183,7 @@ int build_adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj) {
   GARY_CUDA(cudaStreamSynchronize(s));
   const uint32_t words = ((span + 127) / 128) * 4;  // whole quads
   const uint64_t bytes = ((uint64_t)span + nl) * words * 4;
-  size_t free_bytes = 0, total_bytes = 0;
-  GARY_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
-  if (pairs < (g->out_deg_sq - g->dag.m) / 16 || bytes > total_bytes / 8) {
+  if (pairs < (g->out_deg_sq - g->dag.m) / 16 || !room_for_rows(bytes)) {
     adj.low.release();
     return GARY_OK;
   }
@@ -200,7 +200,7 @@ int build_adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj) {
   return GARY_OK;
 }
 
-int build_hub_rows(gary_graph *g, cudaStream_t s, HubRows &hub, DevBuf<uint32_t> &len) {
+int hub_rows(gary_graph *g, cudaStream_t s, HubRows &hub, DevBuf<uint32_t> &len) {
   hub.n_list = 0;
   const uint32_t n = g->n;
   // A union of graphs is ranked graph by graph: its hubs are not the top ids.
@@ -227,20 +227,61 @@ int build_hub_rows(gary_graph *g, cudaStream_t s, HubRows &hub, DevBuf<uint32_t>
                                                  thrust::counting_iterator<uint32_t>(n), hub.list.p,
                                                  IsCounted{g->dag.row.p, len.p}) -
                                  hub.list.p);
-  if ((uint64_t)nl + kHubIds >= (1u << 27)) {  // rows are numbered in 27 bits
+  const uint64_t quads = ((uint64_t)kHubIds + nl) * kHubRowQuads;
+  if ((uint64_t)nl + kHubIds >= (1u << 27) || !room_for_rows(quads * 16)) {  // rows are numbered in 27 bits
     hub.list.release();
     len.release();
     return GARY_OK;
   }
   GARY_TRY(hub.cut.alloc_persistent(nl));
   GARY_TRY(hub.rowof.alloc_persistent(n));
-  GARY_TRY(hub.rows.alloc_persistent(((uint64_t)kHubIds + nl) * kHubRowQuads));
+  GARY_TRY(hub.rows.alloc_persistent(quads));
   GARY_CUDA(cudaMemsetAsync(hub.rowof.p, 0xFF, (uint64_t)n * 4, s));
   k_hub_fill<<<grid_for(((uint64_t)kHubIds + nl) * 32), kThreads, 0, s>>>(
       g->dag.row.p, g->dag.adj.p, len.p, hub.list.p, nl, first, hub.cut.p, hub.rowof.p, hub.rows.p);
   GARY_CUDA(cudaGetLastError());
   hub.n_list = nl;
   hub.first = first;
+  return GARY_OK;
+}
+
+}  // namespace
+
+bool room_for_rows(uint64_t bytes) {
+  size_t free_bytes = 0, total_bytes = 0;
+  if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (bytes > total_bytes / 8) return false;
+  if (bytes > free_bytes / 2) {  // cached blocks may hold the room
+    release_cached_memory();
+    if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+  }
+  return bytes <= free_bytes / 2;
+}
+
+// Rows are an option: where the device has no room for them the plan is made
+// without, as it would be for a graph that rows do not pay for.
+int build_adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj) {
+  const int rc = adj_rows(g, s, adj);
+  if (rc != GARY_ERR_OOM) return rc;
+  GARY_CUDA(cudaStreamSynchronize(s));
+  adj = AdjRows{};
+  clear_error();
+  return GARY_OK;
+}
+
+int build_hub_rows(gary_graph *g, cudaStream_t s, HubRows &hub, DevBuf<uint32_t> &len) {
+  const int rc = hub_rows(g, s, hub, len);
+  if (rc != GARY_ERR_OOM) return rc;
+  GARY_CUDA(cudaStreamSynchronize(s));
+  hub = HubRows{};
+  len.release();
+  clear_error();
   return GARY_OK;
 }
 

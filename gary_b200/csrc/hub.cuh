@@ -74,6 +74,10 @@ constexpr uint32_t kAdjRowIds = 16384;
 // 37.9 ms, RMAT-20 ef5 0.73 / 0.74 / 0.78 / 0.79).
 constexpr uint32_t kAdjMin = 16;
 
+// Rows take at most an eighth of the device's memory and half of what is free, so
+// that the rest of a plan still finds room wherever it did without them.
+bool room_for_rows(uint64_t bytes);
+
 // Builds them when at least an eighth of the pairs of higher neighbours have
 // their second id among the top ids and their first vertex a row; words stays 0
 // otherwise (sparse graphs without hubs: walking lists is cheaper there).

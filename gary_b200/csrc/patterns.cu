@@ -16,9 +16,9 @@
 // consecutive rows, so that their loops have one length, 33.4 ms.)  Then
 //   K4(u) = sum over set bits (i, j) of popcount(row_i AND row_j),
 // since row j holds only positions after j.  Vertices with d <= 128 run on
-// one warp (rows of at most 4 words), d <= 512 on a 256-thread CTA, larger
-// ones on a 1024-thread CTA, with rows in shared memory up to d = 1024 and in
-// a per-CTA HBM buffer beyond.
+// one warp (rows of at most 4 words), d <= 362 on a 256-thread CTA, d <= 877
+// on a 512-thread one, all with rows in shared memory, and larger ones on a
+// 1024-thread CTA with rows in a per-CTA HBM buffer.
 //
 // 4-cycles (symmetric ranked lists): each cycle is counted once at its
 // highest-ranked vertex u, with w the opposite vertex:

@@ -16,7 +16,7 @@ struct PatternPlan {
   DevBuf<Tile> tiles;
   DevBuf<uint32_t> light;    // light vertices (K4 groups index it; C4 warps walk it)
   DevBuf<uint32_t> mid;      // C4: medium vertices, one CTA hash map each; K4: mid vertices
-  DevBuf<uint32_t> big;      // K4: vertices with d+ > 512, largest first (the n_pool with rows in HBM first)
+  DevBuf<uint32_t> big;      // K4: vertices with d+ > 362, largest first (the n_pool with rows in HBM first)
   DevBuf<uint32_t> cursors;  // C4: per window-kernel CTA, 6 x max_pre words of list state; K4: row pool
   AdjRows adj;               // K4: adjacency rows over the top ids
   C4Rows rows;               // C4: the vertices u counted by rows

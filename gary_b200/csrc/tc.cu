@@ -10,8 +10,10 @@
 //     T = sum over v of  sum over in-edges u->v of |S(u,v) & N+(v)|,
 //     S(u,v) = the part of N+(u) after v.
 //
-// One warp (or CTA) holds N+(v) as a shared-memory bitmap (when its id range
-// is short) or hash set, and streams the suffixes S(u,v) of all in-edges of v
+// On skewed graphs the suffix ids among the top 4096 are first taken out and
+// counted by bit rows (hub.cuh).  For the rest, one warp (or CTA) holds N+(v) as
+// a shared-memory bitmap (when its id range is short), hash or pair set
+// (pair_set.cuh; the lists of two octets and less need no set), and streams the suffixes S(u,v) of all in-edges of v
 // with 16-byte loads over the padded lists, all lanes busy.  The probe count
 // is sum over u of C(d+(u), 2), 3.5-4x fewer than streaming N+(v) for every
 // edge (sum of d+(v)) on RMAT graphs, and every read is a coalesced sweep.
@@ -831,9 +833,10 @@ __device__ __forceinline__ uint32_t match_octets(const uint4 &a, const uint4 &b,
 }
 
 // All in-edges of the tiny vertices among 32 light ones (lane's list rv and its
-// nin_v records from ib on, where `tiny`), without a set: the 32 vertices' records are walked flattened, and
-// within a batch of 32 records their octets are, so every lane compares one
-// octet of a suffix with the one or two octets of N+(v).  Building a set costs
+// nin_v records from ib on, where `tiny`), without a set: the 32 vertices'
+// records are walked flattened, and within a batch of 32 records their octets
+// are, so every lane compares one octet of a suffix with the one or two octets
+// of N+(v).  Building a set costs
 // a vertex some thousands of cycles of dependent loads and shared-memory
 // passes whatever its size, which for these vertices is most of their time.
 // All 32 lanes must call.
@@ -966,7 +969,8 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
         const uint32_t *av = g.adj + (uint64_t)rv.x * 4;
         const uint64_t base = inptr[tl.v0];
         const uint32_t lo = av[0];
-        cnt += warp_vertex(g, inedge, tl.v0, VertexHead{rv, lo, av[rv.y - 1] - lo, base + tl.j0, base + tl.j1}, tab, lane, ctl);
+        cnt += warp_vertex(g, inedge, tl.v0,
+                           VertexHead{rv, lo, av[rv.y - 1] - lo, base + tl.j0, base + tl.j1}, tab, lane, ctl);
         continue;
       }
       // a group of light vertices: list positions [v0, v1), 32 ids per load
@@ -984,7 +988,8 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
           gid = g0;
         }
         // the heads of all 32 in lanes, so that the loads a vertex begins with
-        // are waited for once, not by every vertex again
+        // are waited for once, not by every vertex again (batch of 128 graphs
+        // 718 -> 687 us, RMAT-22 ef16 3.04 -> 3.02 ms)
         uint2 rv = make_uint2(0, 0);
         uint64_t kb = 0;
         uint32_t nin = 0;
