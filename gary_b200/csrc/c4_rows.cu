@@ -336,9 +336,7 @@ struct DegreeIn {
 
 }  // namespace
 
-namespace {
-
-int c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
+int build_c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
   const uint32_t n = g->n;
   const uint2 *row = g->sym.row.p;
   const uint32_t *adj = g->sym.adj.p, *dplus = g->dag.outdeg.p;
@@ -391,19 +389,6 @@ int c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
   r.n5 = pick(r.list.p, 2, 31);
   r.n8 = pick(r.list.p + r.n5, 32, 255);
   r.n32 = pick(r.list.p + r.n5 + r.n8, 256, 0xFFFFFFFFu);
-  return GARY_OK;
-}
-
-}  // namespace
-
-int build_c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
-  const int rc = c4_rows(g, s, r);
-  if (rc != GARY_ERR_OOM) return rc;
-  // no room on the device: the wedge kernels take every vertex
-  GARY_CUDA(cudaStreamSynchronize(s));
-  r = C4Rows{};
-  r.lowest = g->n;
-  clear_error();
   return GARY_OK;
 }
 

@@ -158,9 +158,7 @@ __global__ void k_adj_low(const uint2 *__restrict__ row, const uint32_t *__restr
 
 }  // namespace
 
-namespace {
-
-int adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj) {
+int build_adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj) {
   const uint32_t n = g->n, span = std::min(n, kAdjRowIds), first = n - span;
   adj.words = 0;
   if (g->dag.max_len < 3) return GARY_OK;
@@ -200,7 +198,7 @@ int adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj) {
   return GARY_OK;
 }
 
-int hub_rows(gary_graph *g, cudaStream_t s, HubRows &hub, DevBuf<uint32_t> &len) {
+int build_hub_rows(gary_graph *g, cudaStream_t s, HubRows &hub, DevBuf<uint32_t> &len) {
   hub.n_list = 0;
   const uint32_t n = g->n;
   // A union of graphs is ranked graph by graph: its hubs are not the top ids.
@@ -245,9 +243,8 @@ int hub_rows(gary_graph *g, cudaStream_t s, HubRows &hub, DevBuf<uint32_t> &len)
   return GARY_OK;
 }
 
-}  // namespace
-
 bool room_for_rows(uint64_t bytes) {
+  if (bytes <= (1ull << 30)) return true;
   size_t free_bytes = 0, total_bytes = 0;
   if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) {
     cudaGetLastError();
@@ -262,27 +259,6 @@ bool room_for_rows(uint64_t bytes) {
     }
   }
   return bytes <= free_bytes / 2;
-}
-
-// Rows are an option: where the device has no room for them the plan is made
-// without, as it would be for a graph that rows do not pay for.
-int build_adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj) {
-  const int rc = adj_rows(g, s, adj);
-  if (rc != GARY_ERR_OOM) return rc;
-  GARY_CUDA(cudaStreamSynchronize(s));
-  adj = AdjRows{};
-  clear_error();
-  return GARY_OK;
-}
-
-int build_hub_rows(gary_graph *g, cudaStream_t s, HubRows &hub, DevBuf<uint32_t> &len) {
-  const int rc = hub_rows(g, s, hub, len);
-  if (rc != GARY_ERR_OOM) return rc;
-  GARY_CUDA(cudaStreamSynchronize(s));
-  hub = HubRows{};
-  len.release();
-  clear_error();
-  return GARY_OK;
 }
 
 }  // namespace gary

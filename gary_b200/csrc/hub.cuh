@@ -19,6 +19,7 @@
 // above v's own position are read: N+(v) holds no id below v.
 #pragma once
 #include <cstdint>
+#include <new>
 
 #include "graph.cuh"
 #include "internal.cuh"
@@ -74,9 +75,27 @@ constexpr uint32_t kAdjRowIds = 16384;
 // 37.9 ms, RMAT-20 ef5 0.73 / 0.74 / 0.78 / 0.79).
 constexpr uint32_t kAdjMin = 16;
 
-// Rows take at most an eighth of the device's memory and half of what is free, so
-// that the rest of a plan still finds room wherever it did without them.
+// Rows of more than 1 GB take at most an eighth of the device's memory and half of
+// what is free.  (Smaller ones do not ask: the driver's answer takes up to 3 ms,
+// longer than a count of RMAT-20 with its plan.)
 bool room_for_rows(uint64_t bytes);
+
+// Rows are an option: a plan that does not find the memory it needs is made
+// again without them.  build(true) may use rows, build(false) does not.
+template <class F>
+int with_or_without_rows(cudaStream_t s, F build) {
+  int rc;
+  try {
+    rc = build(true);
+  } catch (const std::bad_alloc &) {  // thrust's temporaries (ScratchAlloc)
+    rc = GARY_ERR_OOM;
+  }
+  if (rc != GARY_ERR_OOM) return rc;
+  GARY_CUDA(cudaStreamSynchronize(s));
+  release_cached_memory();
+  clear_error();
+  return build(false);
+}
 
 // Builds them when at least an eighth of the pairs of higher neighbours have
 // their second id among the top ids and their first vertex a row; words stays 0

@@ -1024,13 +1024,15 @@ int c4_win_attr() {
   return GARY_OK;
 }
 
-int build_k4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
+namespace {
+
+int k4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out, bool rows) {
   auto plan = std::make_unique<PatternPlan>();
   const uint32_t n = g->n;
   ScratchAlloc pol_alloc{s};
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
   const uint32_t *dp = g->dag.outdeg.p;
-  GARY_TRY(build_adj_rows(g, s, plan->adj));
+  if (rows) GARY_TRY(build_adj_rows(g, s, plan->adj));
   // warp and mid vertices in id order; big vertices largest first
   GARY_TRY(plan->light.alloc_persistent(std::max<uint32_t>(n, 1)));
   plan->n_light = (uint32_t)(thrust::copy_if(pol, thrust::counting_iterator<uint32_t>(0),
@@ -1065,6 +1067,12 @@ int build_k4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
   GARY_CUDA(cudaStreamSynchronize(s));
   *out = plan.release();
   return GARY_OK;
+}
+
+}  // namespace
+
+int build_k4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
+  return with_or_without_rows(s, [&](bool rows) { return k4_plan(g, s, out, rows); });
 }
 
 int launch_k4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaStream_t s,
@@ -1141,7 +1149,9 @@ int launch_k4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaS
   return GARY_OK;
 }
 
-int build_c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
+namespace {
+
+int c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out, bool rows) {
   GARY_TRY(build_symmetric(g, s));
   auto plan = std::make_unique<PatternPlan>();
   const uint32_t n = g->n;
@@ -1149,7 +1159,8 @@ int build_c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
   DevBuf<uint8_t> cls;
   GARY_TRY(cls.alloc(n, s));
-  GARY_TRY(build_c4_rows(g, s, plan->rows));
+  if (rows) GARY_TRY(build_c4_rows(g, s, plan->rows));
+  else plan->rows.lowest = n;
   k_c4_classify<<<grid_for(n), kThreads, 0, s>>>(g->sym.row.p, g->sym.adj.p, g->dag.outdeg.p, n, plan->rows.lowest,
                                                  (uint32_t)kC4LightWedges, cls.p);
   GARY_CUDA(cudaGetLastError());
@@ -1230,6 +1241,12 @@ int build_c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
   GARY_CUDA(cudaStreamSynchronize(s));
   *out = plan.release();
   return GARY_OK;
+}
+
+}  // namespace
+
+int build_c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
+  return with_or_without_rows(s, [&](bool rows) { return c4_plan(g, s, out, rows); });
 }
 
 int launch_c4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaStream_t s,

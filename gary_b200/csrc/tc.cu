@@ -439,8 +439,10 @@ PlanParams resolve_params(PlanParams pp, uint64_t total_work, uint64_t records) 
   return pp;
 }
 
-int build_k3_plan(gary_graph *g, const PlanParams &pp_in, cudaStream_t s, gary_count_plan **out,
-                  const float *model, bool hubs) {
+namespace {
+
+int k3_plan(gary_graph *g, const PlanParams &pp_in, cudaStream_t s, gary_count_plan **out, const float *model,
+            bool hubs) {
   auto plan = std::make_unique<gary_count_plan>();
   const uint32_t n = g->n;
   ScratchAlloc pol_alloc{s};
@@ -536,6 +538,14 @@ int build_k3_plan(gary_graph *g, const PlanParams &pp_in, cudaStream_t s, gary_c
   tr.mark("tiles");
   *out = plan.release();
   return GARY_OK;
+}
+
+}  // namespace
+
+int build_k3_plan(gary_graph *g, const PlanParams &pp, cudaStream_t s, gary_count_plan **out, const float *model,
+                  bool hubs) {
+  if (!hubs) return k3_plan(g, pp, s, out, model, false);
+  return with_or_without_rows(s, [&](bool rows) { return k3_plan(g, pp, s, out, model, rows); });
 }
 
 // ---------------------------------------------------------------------------
