@@ -161,7 +161,7 @@ __global__ void k_adj_low(const uint2 *__restrict__ row, const uint32_t *__restr
 int build_adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj) {
   const uint32_t n = g->n, span = std::min(n, kAdjRowIds), first = n - span;
   adj.words = 0;
-  if (g->dag.max_len < 3) return GARY_OK;
+  if (g->dag.max_len <= kAdjMaxShort) return GARY_OK;
   ScratchAlloc pol_alloc{s};
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
   DevBuf<unsigned long long> sum;

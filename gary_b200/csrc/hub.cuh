@@ -74,6 +74,10 @@ constexpr uint32_t kAdjRowIds = 16384;
 // Top neighbours a row needs (8 / 16 / 32 / 64: RMAT-22 ef16 33.1 / 33.2 / 33.4 /
 // 37.9 ms, RMAT-20 ef5 0.73 / 0.74 / 0.78 / 0.79).
 constexpr uint32_t kAdjMin = 16;
+// No rows where every list fits one word: they win some 5 us a count and cost 55
+// us in the plan (ER n = 20000, 10 edges a vertex: 52 / 57 us a count, first count
+// with its plan 214 / 157 us, with / without).
+constexpr uint32_t kAdjMaxShort = 32;
 
 // Rows of more than 1 GB take at most an eighth of the device's memory and half of
 // what is free.  (Smaller ones do not ask: the driver's answer takes up to 3 ms,
