@@ -70,73 +70,126 @@ struct MinU64 {
 };
 
 // The records of the padded words w of N+(u): the suffix after v = adj[w], up to
-// len[u] (null: the whole list), keyed by v.  Records are appended tile by tile
-// (in word order within a tile of kCandTile words, one atomic a tile), so the
-// sort that follows moves records only: after hub rows have taken the hub
-// suffixes a third of the words hold one at RMAT-20 ef16.  *cut += the suffix
-// ids past len[u]; *count: the records.
+// len[u] (null: the whole list), keyed by v.  They are written in word order, so
+// that the sort that follows (stable, by v) moves records only (after hub rows
+// have taken the hub suffixes a third of the words hold one at RMAT-20 ef16) and
+// leaves every vertex's records in the same order in every plan of the graph:
+// split vertices are cut by position, and shards of one count come from plans
+// that other processes built.  (Appended in whatever order tiles ran, shards of
+// two plans counted some records twice and others never.)  Two passes, tile by
+// tile: this one marks the words with a record (a bit each, so that d+(v), a
+// scattered read, is not read twice) and counts them: tiles[t], and their sum.  A
+// first count, plan included, takes some 10 us more than with one appending pass
+// (RMAT-16 ef16 0.447 / 0.456 ms, RMAT-20 1.530 / 1.540, RMAT-22 6.03 / 6.05).  total[0] += the suffix ids past
+// len[u], total[1] += the records.
 constexpr int kCandPer = 8;
 constexpr uint32_t kCandTile = kThreads * kCandPer;
+constexpr int kCandWarps = kThreads / 32;
+
+// Suffix ids after position pos of a list cut to `end` ids.
+__device__ __forceinline__ uint32_t kept_suffix(uint32_t end, uint64_t pos) {
+  return end > (uint32_t)pos + 1 ? end - (uint32_t)pos - 1 : 0u;
+}
+
 __global__ void __launch_bounds__(kThreads)
-    k_in_candidates(const uint2 *__restrict__ row, const uint32_t *__restrict__ adj,
-                    const uint32_t *__restrict__ rowid, uint64_t words, const uint32_t *__restrict__ len,
-                    uint32_t *__restrict__ keys, uint2 *__restrict__ vals, unsigned long long *__restrict__ cut,
-                    unsigned long long *__restrict__ count) {
-  constexpr int kW = kThreads / 32;
-  __shared__ uint32_t at[kCandPer * kW];
-  __shared__ unsigned long long s_base;
+    k_in_mark(const uint2 *__restrict__ row, const uint32_t *__restrict__ adj, const uint32_t *__restrict__ rowid,
+              uint64_t words, const uint32_t *__restrict__ len, uint32_t *__restrict__ marks,
+              uint64_t *__restrict__ tiles, unsigned long long *__restrict__ total) {
+  __shared__ uint32_t s_n;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long mine = 0;
-  for (uint64_t t0 = (uint64_t)blockIdx.x * kCandTile; t0 < words; t0 += (uint64_t)gridDim.x * kCandTile) {
-    uint32_t key[kCandPer];
-    uint32_t keep[kCandPer];
-    unsigned has[kCandPer];
+  unsigned long long mine = 0, records = 0;
+  for (uint64_t t = blockIdx.x; t * kCandTile < words; t += gridDim.x) {
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    uint32_t c = 0;
 #pragma unroll
     for (int i = 0; i < kCandPer; ++i) {
-      const uint64_t w = t0 + (uint64_t)i * kThreads + threadIdx.x;
-      key[i] = 0;
-      keep[i] = 0;
+      const uint64_t w = t * kCandTile + (uint64_t)i * kThreads + threadIdx.x;
+      bool has = false;
       if (w < words) {
         const uint32_t u = rowid[w];
         const uint2 r = row[u];
         const uint64_t pos = w - (uint64_t)r.x * 4;
-        if (pos < r.y) {
-          const uint32_t v = adj[w];
-          const uint32_t rem = r.y - (uint32_t)pos - 1;
-          if (rem && row[v].y) {
-            const uint32_t end = len ? len[u] : r.y;
-            keep[i] = end > (uint32_t)pos + 1 ? end - (uint32_t)pos - 1 : 0u;
-            mine += rem - keep[i];
-            key[i] = v;
-          }
+        if (pos + 1 < r.y && row[adj[w]].y) {
+          const uint32_t keep = kept_suffix(len ? len[u] : r.y, pos);
+          mine += r.y - (uint32_t)pos - 1 - keep;
+          has = keep != 0;
         }
       }
-      has[i] = __ballot_sync(kFull, keep[i] != 0);
-      if (lane == 0) at[i * kW + warp] = __popc(has[i]);
+      const unsigned m = __ballot_sync(kFull, has);
+      if (lane == 0) marks[(t * kCandPer + i) * kCandWarps + warp] = m;
+      c += __popc(m);
+    }
+    if (lane == 0) atomicAdd(&s_n, c);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      tiles[t] = s_n;
+      records += s_n;
     }
     __syncthreads();
-    if (warp == 0) {  // where each warp's part of each row of the tile goes
-      uint32_t a = at[2 * lane], b = at[2 * lane + 1];
+  }
+  if (threadIdx.x == 0 && records) atomicAdd(&total[1], records);
+  if (len) {
+    mine = warp_sum_u64(mine);
+    if (lane == 0 && mine) atomicAdd(&total[0], mine);
+  }
+}
+
+// Up to so many tiles, every CTA adds up the counts before its own itself; past
+// them (RMAT-21 and larger) that reads more than a scan's launches cost (a first
+// count with a scan at any size: RMAT-16 0.478 ms, RMAT-20 1.570).
+constexpr uint64_t kCandFewTiles = 1u << 14;
+
+// The second pass writes the marked words' records, a CTA those of consecutive
+// tiles.  tiles: each tile's offset (scanned) or its count.
+__global__ void __launch_bounds__(kThreads)
+    k_in_candidates(const uint2 *__restrict__ row, const uint32_t *__restrict__ adj,
+                    const uint32_t *__restrict__ rowid, uint64_t words, const uint32_t *__restrict__ len,
+                    const uint32_t *__restrict__ marks, const uint64_t *__restrict__ tiles, bool scanned,
+                    uint32_t *__restrict__ keys, uint2 *__restrict__ vals) {
+  __shared__ uint32_t at[kCandPer * kCandWarps];
+  __shared__ unsigned long long s_base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t nt = (words + kCandTile - 1) / kCandTile, per = (nt + gridDim.x - 1) / gridDim.x;
+  const uint64_t t0 = blockIdx.x * per, t1 = min_u64(t0 + per, nt);
+  if (t0 >= t1) return;
+  if (threadIdx.x == 0) s_base = scanned ? tiles[t0] : 0;
+  __syncthreads();
+  if (!scanned) {
+    unsigned long long before = 0;
+    for (uint64_t j = threadIdx.x; j < t0; j += kThreads) before += tiles[j];
+    before = warp_sum_u64(before);
+    if (lane == 0 && before) atomicAdd(&s_base, before);
+    __syncthreads();
+  }
+  for (uint64_t t = t0; t < t1; ++t) {
+    const unsigned long long base = s_base;
+    uint32_t all = 0;  // the tile's records
+    if (warp == 0) {   // where each warp's part of each row of the tile goes
+      const uint32_t *m = marks + t * (kCandPer * kCandWarps);
+      const uint32_t a = __popc(m[2 * lane]), b = __popc(m[2 * lane + 1]);
       const uint32_t incl = warp_inclusive_sum(a + b, lane);
-      if (lane == 31) s_base = atomicAdd(count, (unsigned long long)incl);
       at[2 * lane] = incl - a - b;
       at[2 * lane + 1] = incl - b;
+      all = __shfl_sync(kFull, incl, 31);
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < kCandPer; ++i)
-      if (keep[i]) {
-        const uint64_t o = s_base + at[i * kW + warp] + __popc(has[i] & ((1u << lane) - 1u));
-        keys[o] = key[i];
-        vals[o] = make_uint2((uint32_t)(t0 + (uint64_t)i * kThreads + threadIdx.x + 1), keep[i]);
+    for (int i = 0; i < kCandPer; ++i) {
+      const unsigned m = marks[(t * kCandPer + i) * kCandWarps + warp];
+      if ((m >> lane) & 1u) {
+        const uint64_t w = t * kCandTile + (uint64_t)i * kThreads + threadIdx.x;
+        const uint32_t u = rowid[w];
+        const uint2 r = row[u];
+        const uint64_t o = base + at[i * kCandWarps + warp] + __popc(m & ((1u << lane) - 1u));
+        keys[o] = adj[w];
+        vals[o] = make_uint2((uint32_t)(w + 1), kept_suffix(len ? len[u] : r.y, w - (uint64_t)r.x * 4));
       }
+    }
+    if (threadIdx.x == 0) s_base = base + all;
     __syncthreads();
   }
-  static_assert(kCandPer * kW == 64, "two entries a lane");
-  if (len) {
-    mine = warp_sum_u64(mine);
-    if (lane == 0 && mine) atomicAdd(cut, mine);
-  }
+  static_assert(kCandPer * kCandWarps == 64, "two entries a lane");
 }
 
 __global__ void k_in_heads(const uint32_t *__restrict__ keys, uint64_t m,
@@ -356,22 +409,32 @@ int build_in_index(gary_graph *g, cudaStream_t s, const DevBuf<uint32_t> &len, I
   DevBuf<uint2> vals, vals2;
   uint64_t m = 0;
   {
-    DevBuf<uint32_t> rowid;
-    DevBuf<unsigned long long> cut;  // {suffix ids cut off, records}
-    GARY_TRY(cut.alloc(2, s));
-    GARY_CUDA(cudaMemsetAsync(cut.p, 0, 16, s));
+    DevBuf<uint32_t> rowid, marks;
+    DevBuf<uint64_t> tiles;
+    DevBuf<unsigned long long> total;  // {suffix ids cut off, records}
+    const uint64_t nt = (W + kCandTile - 1) / kCandTile;
+    const bool scan = nt > kCandFewTiles;
+    GARY_TRY(total.alloc(2, s));
+    GARY_CUDA(cudaMemsetAsync(total.p, 0, 16, s));
+    GARY_TRY(tiles.alloc(std::max<uint64_t>(nt, 1), s));
+    GARY_TRY(marks.alloc(std::max<uint64_t>(nt * kCandPer * kCandWarps, 1), s));
     GARY_TRY(padded_rowid(g->dag, rowid, s));
-    GARY_TRY(keys.alloc(std::max<uint64_t>(W, 1), s));
-    GARY_TRY(vals.alloc(std::max<uint64_t>(W, 1), s));
+    const unsigned grid = grid_for(nt * kThreads);
     if (W)
-      k_in_candidates<<<grid_for((W + kCandPer - 1) / kCandPer), kThreads, 0, s>>>(
-          g->dag.row.p, g->dag.adj.p, rowid.p, W, len.p, keys.p, vals.p, cut.p, cut.p + 1);
+      k_in_mark<<<grid, kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, len.p, marks.p, tiles.p, total.p);
     GARY_CUDA(cudaGetLastError());
+    if (scan) thrust::exclusive_scan(pol, tiles.p, tiles.p + nt, tiles.p, (uint64_t)0);
     unsigned long long h[2] = {0, 0};
-    GARY_CUDA(cudaMemcpyAsync(h, cut.p, 16, cudaMemcpyDeviceToHost, s));
+    GARY_CUDA(cudaMemcpyAsync(h, total.p, 16, cudaMemcpyDeviceToHost, s));
     GARY_CUDA(cudaStreamSynchronize(s));
     in.hub_work = h[0];
     m = h[1];
+    GARY_TRY(keys.alloc(std::max<uint64_t>(m, 1), s));
+    GARY_TRY(vals.alloc(std::max<uint64_t>(m, 1), s));
+    if (m)
+      k_in_candidates<<<grid, kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, len.p, marks.p, tiles.p, scan,
+                                                keys.p, vals.p);
+    GARY_CUDA(cudaGetLastError());
   }
   if (m) {
     GARY_TRY(keys2.alloc(m, s));
