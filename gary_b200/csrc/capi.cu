@@ -3,6 +3,7 @@
 // to a GARY_ERR_* status (the reference's checkCudaErrors exits the process
 // instead, common/HelperCUDA.h:582-595).
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstdarg>
 #include <cstdio>
@@ -124,9 +125,21 @@ void trim_blocks_locked(int d, uint64_t keep) {
   }
   if (cur != d) cudaSetDevice(cur);
 }
+
+// Tuning key "refuse_block": the k-th block asked for from then on is refused as
+// a full device would refuse it (0: none), so that tests reach what a call leaves
+// behind when it runs out of memory.
+std::atomic<uint64_t> g_refuse_block{0};
+bool refuse_block() {
+  uint64_t k = g_refuse_block.load(std::memory_order_relaxed);
+  while (k && !g_refuse_block.compare_exchange_weak(k, k - 1, std::memory_order_relaxed)) {
+  }
+  return k == 1;
+}
 }  // namespace
 
 cudaError_t persistent_alloc(void **p, size_t bytes) {
+  if (refuse_block()) return cudaErrorMemoryAllocation;
   const int d = device_ordinal();
   const size_t rb = round_block(bytes);
   if (d >= 0 && d < 64) {
@@ -438,6 +451,7 @@ extern "C" int gary_tune(const char *key, uint64_t value) {
   else if (k == "vertex_overhead") p.vertex_overhead = value;
   else if (k == "min_blocks" && (value == 0 || value == 2 || value == 3)) p.min_blocks = (uint32_t)value;
   else if (k == "pool_keep_bytes") gary::set_pool_keep_bytes(value);
+  else if (k == "refuse_block") gary::g_refuse_block = value;
   else if (k == "reset") p = gary::PlanParams{};
   else {
     gary::set_error("unknown tuning key '%s' or value %llu out of range", key,

@@ -1398,8 +1398,12 @@ int build_symmetric(gary_graph *g, cudaStream_t s) {
     GARY_TRY(alt.alloc(std::max<uint64_t>(m2, 1), s));
     if (m2) GARY_TRY(radix_sort_keys(keys, alt, m2, 2 * lg, s));
   }
-  GARY_TRY(padded_from_keys(keys, m2, n, lg, g->sym, s));
+  // only whole lists become the graph's: a build that ends early (no memory for
+  // one of the arrays) is begun anew by the next call, not taken for complete
+  PaddedCSR sym;
+  GARY_TRY(padded_from_keys(keys, m2, n, lg, sym, s));
   GARY_CUDA(cudaStreamSynchronize(s));
+  g->sym = std::move(sym);
   return GARY_OK;
 }
 

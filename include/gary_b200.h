@@ -255,6 +255,10 @@ int gary_gen_ba(uint32_t n, uint32_t m, uint64_t seed, uint32_t *src, uint32_t *
  *                     a caching allocator, so a repeated upload makes no
  *                     driver allocation call; 0 returns both now and at
  *                     every later free or sync); "reset" leaves it alone
+ *   "refuse_block"    k: the k-th device block (an array that outlives its
+ *                     call) allocated from now on is refused once, as by a
+ *                     full device; 0 (the default): none.  For tests; "reset"
+ *                     leaves it alone
  *   "reset"           restore every plan default
  * No reference counterpart: the reference fixes its launch shape in each test
  * (test/TriQueryTest.cu:98-99, 116-117). */
