@@ -336,12 +336,14 @@ struct DegreeIn {
 
 }  // namespace
 
-int build_c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
+int build_c4_rows(gary_graph *g, cudaStream_t s, Rows use, C4Rows &r) {
   const uint32_t n = g->n;
   const uint2 *row = g->sym.row.p;
   const uint32_t *adj = g->sym.adj.p, *dplus = g->dag.outdeg.p;
   r.slabs = 0;
   r.lowest = n;
+  r.shared = use != Rows::kNone;
+  if (use == Rows::kNone) return GARY_OK;
   ScratchAlloc pol_alloc{s};
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
   SlabEnds se{};
@@ -356,6 +358,7 @@ int build_c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
   GARY_CUDA(cudaMemcpyAsync(h, stat.p, sizeof(h), cudaMemcpyDeviceToHost, s));
   GARY_CUDA(cudaStreamSynchronize(s));
   uint64_t used = 0;  // by all slabs' rows
+  const uint64_t shard_most = std::max(kC4ShardWordBytes * g->dag.words, kC4ShardLeast);
   DevBuf<uint32_t> list;
   GARY_TRY(list.alloc(n, s));
   for (int k = 0; k < se.slabs && h[k] && h[k] / kC4RowWedges >= h[kC4MaxSlabs]; ++k) {
@@ -367,7 +370,11 @@ int build_c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r) {
                                                    thrust::counting_iterator<uint32_t>(n), list.p,
                                                    TouchesSlab{row, adj, sl.first, sl.end}) - list.p);
     const uint64_t bytes = ((uint64_t)span + nl + 1) * kC4RowQuads * 16;
-    if (!room_for_rows(used + bytes)) break;
+    const bool in_shards = used + bytes <= shard_most;
+    const bool take = use == Rows::kRequired ? in_shards : room_for_rows(used + bytes);
+    // both kinds of plan have this slab
+    r.shared = r.shared && take && in_shards;
+    if (!take) break;
     used += bytes;
     GARY_TRY(sl.rowof.alloc_persistent(n));
     GARY_TRY(sl.rows.alloc_persistent(bytes / 16));

@@ -19,6 +19,7 @@
 #include <cstdint>
 
 #include "graph.cuh"
+#include "hub.cuh"
 #include "internal.cuh"
 
 namespace gary {
@@ -32,6 +33,12 @@ constexpr int kC4MaxSlabs = 8;
 // without rows 16.4 and 142.7).
 constexpr uint64_t kC4RowWedges = 10;
 
+// A shard's slabs take at most so many bytes per padded word of the graph's lists,
+// or 128 MB.  The symmetric lists' own build takes more (two arrays of two 8-byte
+// keys a word), so a shard is not refused for its rows on a device that could hold
+// the lists.
+constexpr uint64_t kC4ShardWordBytes = 24, kC4ShardLeast = 128u << 20;
+
 // Rows over the ids [first, end): row p < end - first holds the neighbours of
 // first + p above it, the rows after those (rowof) all of an x's below `first`.
 struct C4Slab {
@@ -44,6 +51,7 @@ struct C4Rows {
   C4Slab slab[kC4MaxSlabs];
   int slabs = 0;
   uint32_t lowest = 0;     // the wedge kernels take the u below
+  bool shared = false;     // shards and whole counts have these same slabs
   // vertices w of two neighbours and more, by the counters their degree needs:
   // 5 and 8 slices in a warp's registers, and shared 32-bit counters of a CTA
   DevBuf<uint32_t> list;
@@ -51,8 +59,9 @@ struct C4Rows {
   DevBuf<uint32_t> queue;            // three words a slab
 };
 
-// Builds the slabs that pay (none: slabs 0, lowest n).
-int build_c4_rows(gary_graph *g, cudaStream_t s, C4Rows &r);
+// Builds the slabs that pay (none: slabs 0, lowest n): for a whole count those
+// there is room for, for a shard (Rows::kRequired) those within kC4ShardWordBytes.
+int build_c4_rows(gary_graph *g, cudaStream_t s, Rows use, C4Rows &r);
 
 // Adds this shard's cycles to *d_out.
 int launch_c4_rows(gary_graph *g, const C4Rows &r, unsigned long long *d_out, cudaStream_t s, uint32_t shard,

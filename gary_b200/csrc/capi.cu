@@ -334,7 +334,8 @@ void free_plans(gary_graph *g) {
   }
   delete g->k4_plan;
   delete g->c4_plan;
-  g->k4_plan = g->c4_plan = nullptr;
+  delete g->c4_shard_plan;
+  g->k4_plan = g->c4_plan = g->c4_shard_plan = nullptr;
 }
 
 namespace {
@@ -357,6 +358,7 @@ int guarded(const char *what, F &&f) {
 }
 
 int plan_slot(int pattern, int sched) { return (pattern - 3) * 2 + sched; }
+constexpr int kShardSlot = 2;    // + sched: a shard's plan where the whole count's had no room for rows
 constexpr int kProfileSlot = 7;  // the plan of gary_tc_features and gary_tc_profile: no hub rows
 
 PlanParams g_tuning;  // process-wide knobs of the counting plans (gary_tune)
@@ -376,6 +378,8 @@ int count_async(gary_graph *g, int pattern, int sched, cudaStream_t s, unsigned 
   GARY_CHECK_ARG(sched == GARY_SCHED_PLAIN || sched == GARY_SCHED_LEARNED, "unknown scheduler %d",
                  sched);
   GARY_CHECK_ARG(nshards >= 1 && shard < nshards, "shard %u of %u is out of range", shard, nshards);
+  // what a shard covers must not depend on this device's free memory
+  const Rows rows = nshards > 1 ? Rows::kRequired : Rows::kOptional;
   if (own_word && pattern != GARY_PATTERN_TRIANGLE) {
     if (!g->result.p) GARY_TRY(g->result.alloc_persistent(1));
     d_out = g->result.p;
@@ -390,10 +394,16 @@ int count_async(gary_graph *g, int pattern, int sched, cudaStream_t s, unsigned 
     return launch_k4(g, g->k4_plan, d_out, s, shard, nshards);
   }
   if (pattern == GARY_PATTERN_4CYCLE) {
-    if (!g->c4_plan) GARY_TRY(build_c4_plan(g, s, &g->c4_plan));
-    return launch_c4(g, g->c4_plan, d_out, s, shard, nshards);
+    PatternPlan *plan = nshards > 1 ? g->c4_shard_plan : g->c4_plan;
+    if (nshards > 1 && g->c4_plan && g->c4_plan->rows.shared) plan = g->c4_plan;
+    if (!plan) {
+      GARY_TRY(build_c4_plan(g, s, &plan, rows));
+      (nshards > 1 && (g->c4_plan || !plan->rows.shared) ? g->c4_shard_plan : g->c4_plan) = plan;
+    }
+    return launch_c4(g, plan, d_out, s, shard, nshards);
   }
-  const int slot = plan_slot(pattern, sched);
+  int slot = plan_slot(pattern, sched);
+  if (nshards > 1 && g->plans[slot] && !g->plans[slot]->rows_by_graph) slot = kShardSlot + sched;
   if (!g->plans[slot]) {
     if (sched == GARY_SCHED_LEARNED) {
       std::vector<float> model;
@@ -405,9 +415,9 @@ int count_async(gary_graph *g, int pattern, int sched, cudaStream_t s, unsigned 
         set_error("GARY_SCHED_LEARNED needs a cost model: call gary_set_cost_model first");
         return GARY_ERR_INVALID;
       }
-      GARY_TRY(build_k3_plan(g, tuned_params(), s, &g->plans[slot], model.data()));
+      GARY_TRY(build_k3_plan(g, tuned_params(), s, &g->plans[slot], model.data(), rows));
     } else {
-      GARY_TRY(build_k3_plan(g, tuned_params(), s, &g->plans[slot]));
+      GARY_TRY(build_k3_plan(g, tuned_params(), s, &g->plans[slot], nullptr, rows));
     }
   }
   return launch_k3(g, g->plans[slot], d_out, s, shard, nshards);
@@ -476,7 +486,7 @@ extern "C" int gary_tc_features(gary_graph *g, float *d_x, uint8_t *d_legal, voi
   return guarded("gary_tc_features", [&] {
     cudaStream_t s = gary::as_stream(stream);
     const int slot = gary::kProfileSlot;
-    if (!g->plans[slot]) GARY_TRY(gary::build_k3_plan(g, gary::tuned_params(), s, &g->plans[slot], nullptr, false));
+    if (!g->plans[slot]) GARY_TRY(gary::build_k3_plan(g, gary::tuned_params(), s, &g->plans[slot], nullptr, gary::Rows::kNone));
     return gary::k3_features(g, g->plans[slot], d_x, d_legal, s);
   });
 }
@@ -488,7 +498,7 @@ extern "C" int gary_tc_profile(gary_graph *g, int variant, uint64_t *d_cycles, u
   return guarded("gary_tc_profile", [&] {
     cudaStream_t s = gary::as_stream(stream);
     const int slot = gary::kProfileSlot;
-    if (!g->plans[slot]) GARY_TRY(gary::build_k3_plan(g, gary::tuned_params(), s, &g->plans[slot], nullptr, false));
+    if (!g->plans[slot]) GARY_TRY(gary::build_k3_plan(g, gary::tuned_params(), s, &g->plans[slot], nullptr, gary::Rows::kNone));
     gary::DevBuf<uint8_t> forced;
     if (variant >= 0) {
       GARY_TRY(forced.alloc(g->n, s));

@@ -71,6 +71,7 @@ struct gary_graph {
   gary_count_plan *plans[8] = {nullptr};
   gary::PatternPlan *k4_plan = nullptr;
   gary::PatternPlan *c4_plan = nullptr;
+  gary::PatternPlan *c4_shard_plan = nullptr;  // where shards cannot share c4_plan (C4Rows::shared)
   gary::DevBuf<unsigned long long> result;  // device word for gary_count
   gary_count_stats last{};
   bool last_timed = false;  // ev0/ev1 bracket the last counting kernel

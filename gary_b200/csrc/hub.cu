@@ -198,8 +198,9 @@ int build_adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj) {
   return GARY_OK;
 }
 
-int build_hub_rows(gary_graph *g, cudaStream_t s, HubRows &hub, DevBuf<uint32_t> &len) {
+int build_hub_rows(gary_graph *g, cudaStream_t s, Rows use, HubRows &hub, DevBuf<uint32_t> &len) {
   hub.n_list = 0;
+  if (use == Rows::kNone) return GARY_OK;
   const uint32_t n = g->n;
   // A union of graphs is ranked graph by graph: its hubs are not the top ids.
   if (n <= 2 * kHubIds || g->ngroups || g->dag.max_len < kHubMin) return GARY_OK;
@@ -226,7 +227,9 @@ int build_hub_rows(gary_graph *g, cudaStream_t s, HubRows &hub, DevBuf<uint32_t>
                                                  IsCounted{g->dag.row.p, len.p}) -
                                  hub.list.p);
   const uint64_t quads = ((uint64_t)kHubIds + nl) * kHubRowQuads;
-  if ((uint64_t)nl + kHubIds >= (1u << 27) || !room_for_rows(quads * 16)) {  // rows are numbered in 27 bits
+  const bool fits = (uint64_t)nl + kHubIds < (1u << 27);  // rows are numbered in 27 bits
+  if (!fits || (use == Rows::kOptional && !room_for_rows(quads * 16))) {
+    hub.no_room = fits;
     hub.list.release();
     len.release();
     return GARY_OK;

@@ -47,6 +47,7 @@ struct HubRows {
   DevBuf<uint32_t> cut;    // per listed vertex: where its counted ids begin in N+(u), a multiple of 8
   uint32_t n_list = 0;     // 0: the plan has no hub rows
   uint32_t first = 0;      // n - kHubIds
+  bool no_room = false;    // n_list is 0 for want of memory
 };
 
 struct HubView {
@@ -84,13 +85,20 @@ constexpr uint32_t kAdjMaxShort = 32;
 // longer than a count of RMAT-20 with its plan.)
 bool room_for_rows(uint64_t bytes);
 
-// Rows are an option: a plan that does not find the memory it needs is made
-// again without them.  build(true) may use rows, build(false) does not.
+// Whether a plan has rows.  In the plans of triangles and 4-cycles rows decide
+// which part of the count a shard is, and the shards of one count come from plans
+// that several processes built, each on a device of its own.  So the plan of a
+// shard has the rows that the graph alone decides on (kRequired) or ends with
+// GARY_ERR_OOM; the plan of a whole count has them where there is room (kOptional).
+enum class Rows { kNone, kOptional, kRequired };
+
+// For a whole count rows are an option: a plan that does not find the memory it
+// needs is made again without them.
 template <class F>
 int with_or_without_rows(cudaStream_t s, F build) {
   int rc;
   try {
-    rc = build(true);
+    rc = build(Rows::kOptional);
   } catch (const std::bad_alloc &) {  // thrust's temporaries (ScratchAlloc)
     rc = GARY_ERR_OOM;
   }
@@ -98,7 +106,7 @@ int with_or_without_rows(cudaStream_t s, F build) {
   GARY_CUDA(cudaStreamSynchronize(s));
   release_cached_memory();
   clear_error();
-  return build(false);
+  return build(Rows::kNone);
 }
 
 // Builds them when at least an eighth of the pairs of higher neighbours have
@@ -108,8 +116,11 @@ int build_adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj);
 
 // Builds the rows of g's DAG when they pay, and len[u], the part of N+(u) the
 // middle-vertex walk still covers (all of it for a vertex not counted here).
-// Otherwise leaves hub.n_list 0 and len empty.
-int build_hub_rows(gary_graph *g, cudaStream_t s, HubRows &hub, DevBuf<uint32_t> &len);
+// Otherwise leaves hub.n_list 0 and len empty; hub.no_room says that they would
+// have paid.  (Required rows do not ask for room: a row of 512 bytes takes 57 ids
+// or more out of the walk, and each of them saves the plan 24 bytes of records to
+// sort.)
+int build_hub_rows(gary_graph *g, cudaStream_t s, Rows use, HubRows &hub, DevBuf<uint32_t> &len);
 
 // The bits of word `word` (of a row) from bit position `from` on.
 __device__ __forceinline__ uint32_t bits_from(uint32_t x, uint32_t word, uint32_t from) {

@@ -1026,13 +1026,13 @@ int c4_win_attr() {
 
 namespace {
 
-int k4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out, bool rows) {
+int k4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out, Rows rows) {
   auto plan = std::make_unique<PatternPlan>();
   const uint32_t n = g->n;
   ScratchAlloc pol_alloc{s};
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
   const uint32_t *dp = g->dag.outdeg.p;
-  if (rows) GARY_TRY(build_adj_rows(g, s, plan->adj));
+  if (rows != Rows::kNone) GARY_TRY(build_adj_rows(g, s, plan->adj));
   // warp and mid vertices in id order; big vertices largest first
   GARY_TRY(plan->light.alloc_persistent(std::max<uint32_t>(n, 1)));
   plan->n_light = (uint32_t)(thrust::copy_if(pol, thrust::counting_iterator<uint32_t>(0),
@@ -1072,7 +1072,8 @@ int k4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out, bool rows) {
 }  // namespace
 
 int build_k4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
-  return with_or_without_rows(s, [&](bool rows) { return k4_plan(g, s, out, rows); });
+  // the classes go by degree alone, so a shard is the same with rows and without
+  return with_or_without_rows(s, [&](Rows rows) { return k4_plan(g, s, out, rows); });
 }
 
 int launch_k4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaStream_t s,
@@ -1151,7 +1152,7 @@ int launch_k4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaS
 
 namespace {
 
-int c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out, bool rows) {
+int c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out, Rows rows) {
   GARY_TRY(build_symmetric(g, s));
   auto plan = std::make_unique<PatternPlan>();
   const uint32_t n = g->n;
@@ -1159,8 +1160,7 @@ int c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out, bool rows) {
   auto pol = thrust::cuda::par_nosync(pol_alloc).on(s);
   DevBuf<uint8_t> cls;
   GARY_TRY(cls.alloc(n, s));
-  if (rows) GARY_TRY(build_c4_rows(g, s, plan->rows));
-  else plan->rows.lowest = n;
+  GARY_TRY(build_c4_rows(g, s, rows, plan->rows));
   k_c4_classify<<<grid_for(n), kThreads, 0, s>>>(g->sym.row.p, g->sym.adj.p, g->dag.outdeg.p, n, plan->rows.lowest,
                                                  (uint32_t)kC4LightWedges, cls.p);
   GARY_CUDA(cudaGetLastError());
@@ -1245,8 +1245,9 @@ int c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out, bool rows) {
 
 }  // namespace
 
-int build_c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out) {
-  return with_or_without_rows(s, [&](bool rows) { return c4_plan(g, s, out, rows); });
+int build_c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out, Rows rows) {
+  if (rows != Rows::kOptional) return c4_plan(g, s, out, rows);
+  return with_or_without_rows(s, [&](Rows use) { return c4_plan(g, s, out, use); });
 }
 
 int launch_c4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaStream_t s,

@@ -31,7 +31,7 @@ struct PatternPlan {
 int build_k4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out);
 int launch_k4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaStream_t s,
               uint32_t shard, uint32_t nshards);
-int build_c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out);
+int build_c4_plan(gary_graph *g, cudaStream_t s, PatternPlan **out, Rows rows);
 int launch_c4(gary_graph *g, PatternPlan *plan, unsigned long long *d_out, cudaStream_t s,
               uint32_t shard, uint32_t nshards);
 

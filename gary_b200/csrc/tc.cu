@@ -505,7 +505,7 @@ PlanParams resolve_params(PlanParams pp, uint64_t total_work, uint64_t records) 
 namespace {
 
 int k3_plan(gary_graph *g, const PlanParams &pp_in, cudaStream_t s, gary_count_plan **out, const float *model,
-            bool hubs) {
+            Rows rows) {
   auto plan = std::make_unique<gary_count_plan>();
   const uint32_t n = g->n;
   ScratchAlloc pol_alloc{s};
@@ -513,7 +513,8 @@ int k3_plan(gary_graph *g, const PlanParams &pp_in, cudaStream_t s, gary_count_p
   PhaseTrace tr("triangle plan", s);
   {
     DevBuf<uint32_t> len;
-    if (hubs) GARY_TRY(build_hub_rows(g, s, plan->hub, len));
+    GARY_TRY(build_hub_rows(g, s, rows, plan->hub, len));
+    plan->rows_by_graph = rows != Rows::kNone && !plan->hub.no_room;
     tr.mark("hub rows");
     GARY_TRY(build_in_index(g, s, len, plan->in));
   }
@@ -606,9 +607,9 @@ int k3_plan(gary_graph *g, const PlanParams &pp_in, cudaStream_t s, gary_count_p
 }  // namespace
 
 int build_k3_plan(gary_graph *g, const PlanParams &pp, cudaStream_t s, gary_count_plan **out, const float *model,
-                  bool hubs) {
-  if (!hubs) return k3_plan(g, pp, s, out, model, false);
-  return with_or_without_rows(s, [&](bool rows) { return k3_plan(g, pp, s, out, model, rows); });
+                  Rows rows) {
+  if (rows != Rows::kOptional) return k3_plan(g, pp, s, out, model, rows);
+  return with_or_without_rows(s, [&](Rows use) { return k3_plan(g, pp, s, out, model, use); });
 }
 
 // ---------------------------------------------------------------------------

@@ -125,6 +125,8 @@ struct gary_count_plan {
   gary::PlanParams params;
   gary::InIndex in;
   gary::HubRows hub;
+  // hub rows, or none, as the graph alone decides: every shard needs such a plan
+  bool rows_by_graph = false;
   gary::DevBuf<uint8_t> vclass;
   gary::DevBuf<uint32_t> light;  // light vertices (group tiles index this list)
   uint32_t n_light = 0;
@@ -141,10 +143,10 @@ struct gary_count_plan {
 
 namespace gary {
 // model: host copy of a cost-model parameter block (learned plan) or null.
-// hubs: false keeps every suffix whole in the middle-vertex walk (the plan the
+// rows: kNone keeps every suffix whole in the middle-vertex walk (the plan the
 // cost model's features and cycle logs are taken on).
 int build_k3_plan(gary_graph *g, const PlanParams &pp, cudaStream_t s, gary_count_plan **out,
-                  const float *model = nullptr, bool hubs = true);
+                  const float *model = nullptr, Rows rows = Rows::kOptional);
 // Cost-model features and legal-variant masks of every middle vertex.
 int k3_features(gary_graph *g, gary_count_plan *plan, float *d_x, uint8_t *d_legal, cudaStream_t s);
 // d_out null: the count goes to the plan's own SchedState::total.

@@ -154,7 +154,10 @@ int gary_count_status(gary_graph *g, void *stream);
 
 /* One shard of the count: every rank holds the whole graph and counts tile
  * ranges [shard/nshards, (shard+1)/nshards) of the plan; the shard totals sum
- * to the full count.  No reference counterpart (the reference is single-GPU,
+ * to the full count, also where every shard is counted by a process and on a
+ * device of its own (devices of one kind, the same tuning and cost model): what
+ * a shard covers depends on the graph, not on the memory that is free.  Where
+ * that does not suffice, the call returns GARY_ERR_OOM.  No reference counterpart (the reference is single-GPU,
  * src/DeviceGraph.cu:91-96). */
 int gary_count_shard_async(gary_graph *g, int pattern, int sched, uint32_t shard,
                            uint32_t nshards, void *stream, uint64_t *d_out);
