@@ -35,6 +35,7 @@
 
 #include <algorithm>
 #include <memory>
+#include <numeric>
 
 #include "bulk.cuh"
 #include "mlp.cuh"
@@ -70,18 +71,19 @@ struct MinU64 {
 };
 
 // The records of the padded words w of N+(u): the suffix after v = adj[w], up to
-// len[u] (null: the whole list), keyed by v.  They are written in word order, so
-// that the sort that follows (stable, by v) moves records only (after hub rows
-// have taken the hub suffixes a third of the words hold one at RMAT-20 ef16) and
-// leaves every vertex's records in the same order in every plan of the graph:
-// split vertices are cut by position, and shards of one count come from plans
-// that other processes built.  (Appended in whatever order tiles ran, shards of
-// two plans counted some records twice and others never.)  Two passes, tile by
-// tile: this one marks the words with a record (a bit each, so that d+(v), a
-// scattered read, is not read twice) and counts them: tiles[t], and their sum.  A
-// first count, plan included, takes some 10 us more than with one appending pass
-// (RMAT-16 ef16 0.447 / 0.456 ms, RMAT-20 1.530 / 1.540, RMAT-22 6.03 / 6.05).  total[0] += the suffix ids past
-// len[u], total[1] += the records.
+// len[u] (null: the whole list), keyed by v.  They are written in an order that
+// follows from the lists' size alone (tile_stride), so that the sort after it
+// (stable, by v) moves records only (with hub rows a third of the words hold one at
+// RMAT-20 ef16) and leaves every vertex's records in the same order in every plan
+// of the graph: split vertices are cut by position, and shards of one count come
+// from plans that other processes built.  (Appended in whatever order tiles ran,
+// shards of two plans counted some records twice and others never.)
+// Two passes, tile by tile of kCandTile words.  This one marks the words with a
+// record, a bit each, so that d+(v), a scattered read, is not read twice, and
+// counts them: tiles[q] of the q-th tile.  total[0] += the suffix ids past len[u],
+// total[1] += the records.  A first count, plan included, takes some 10 us more
+// than with one appending pass (RMAT-16 ef16 0.447 / 0.456 ms, RMAT-20 1.530 /
+// 1.540, RMAT-22 6.03 / 6.05).
 constexpr int kCandPer = 8;
 constexpr uint32_t kCandTile = kThreads * kCandPer;
 constexpr int kCandWarps = kThreads / 32;
@@ -93,12 +95,14 @@ __device__ __forceinline__ uint32_t kept_suffix(uint32_t end, uint64_t pos) {
 
 __global__ void __launch_bounds__(kThreads)
     k_in_mark(const uint2 *__restrict__ row, const uint32_t *__restrict__ adj, const uint32_t *__restrict__ rowid,
-              uint64_t words, const uint32_t *__restrict__ len, uint32_t *__restrict__ marks,
+              uint64_t words, uint64_t stride, const uint32_t *__restrict__ len, uint32_t *__restrict__ marks,
               uint64_t *__restrict__ tiles, unsigned long long *__restrict__ total) {
   __shared__ uint32_t s_n;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long mine = 0, records = 0;
-  for (uint64_t t = blockIdx.x; t * kCandTile < words; t += gridDim.x) {
+  const uint64_t nt = (words + kCandTile - 1) / kCandTile;
+  for (uint64_t q = blockIdx.x; q < nt; q += gridDim.x) {
+    const uint64_t t = q * stride % nt;
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
     uint32_t c = 0;
@@ -123,7 +127,7 @@ __global__ void __launch_bounds__(kThreads)
     if (lane == 0) atomicAdd(&s_n, c);
     __syncthreads();
     if (threadIdx.x == 0) {
-      tiles[t] = s_n;
+      tiles[q] = s_n;
       records += s_n;
     }
     __syncthreads();
@@ -135,17 +139,30 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// Tile q of the record order is tile q * stride mod nt of the words.  From 2^16
+// tiles (512 MB of lists, four times the L2) consecutive tiles come from all over
+// the graph, smaller lists are taken in word order: ms a count appended as before /
+// in word order / strided, RMAT-24 ef32 64.2 / 65.0 / 61.7, RMAT-24 ef16 20.08 /
+// 20.22 / 19.98, RMAT-23 ef16 7.85 / 7.87 / 7.78; RMAT-22 ef32 8.65 / 8.62 / 8.67,
+// RMAT-22 ef16 3.010 / 3.020 / 3.059, RMAT-20 0.512 / 0.511 / 0.513.
+uint64_t tile_stride(uint64_t nt) {
+  if (nt < (1u << 16)) return 1;
+  uint64_t k = (uint64_t)(0.6180339887 * (double)nt) | 1;  // golden section: even spread
+  while (std::gcd(k, nt) != 1) k += 2;
+  return k;
+}
+
 // Up to so many tiles, every CTA adds up the counts before its own itself; past
 // them (RMAT-21 and larger) that reads more than a scan's launches cost (a first
 // count with a scan at any size: RMAT-16 0.478 ms, RMAT-20 1.570).
 constexpr uint64_t kCandFewTiles = 1u << 14;
 
-// The second pass writes the marked words' records, a CTA those of consecutive
-// tiles.  tiles: each tile's offset (scanned) or its count.
+// The second pass writes the marked words' records, a CTA those of tiles that
+// follow one another in the order.  tiles: each tile's offset (scanned) or its count.
 __global__ void __launch_bounds__(kThreads)
     k_in_candidates(const uint2 *__restrict__ row, const uint32_t *__restrict__ adj,
-                    const uint32_t *__restrict__ rowid, uint64_t words, const uint32_t *__restrict__ len,
-                    const uint32_t *__restrict__ marks, const uint64_t *__restrict__ tiles, bool scanned,
+                    const uint32_t *__restrict__ rowid, uint64_t words, uint64_t stride,
+                    const uint32_t *__restrict__ len, const uint32_t *__restrict__ marks, const uint64_t *__restrict__ tiles, bool scanned,
                     uint32_t *__restrict__ keys, uint2 *__restrict__ vals) {
   __shared__ uint32_t at[kCandPer * kCandWarps];
   __shared__ unsigned long long s_base;
@@ -162,7 +179,8 @@ __global__ void __launch_bounds__(kThreads)
     if (lane == 0 && before) atomicAdd(&s_base, before);
     __syncthreads();
   }
-  for (uint64_t t = t0; t < t1; ++t) {
+  for (uint64_t q = t0; q < t1; ++q) {
+    const uint64_t t = q * stride % nt;
     const unsigned long long base = s_base;
     uint32_t all = 0;  // the tile's records
     if (warp == 0) {   // where each warp's part of each row of the tile goes
@@ -414,6 +432,7 @@ int build_in_index(gary_graph *g, cudaStream_t s, const DevBuf<uint32_t> &len, I
     DevBuf<unsigned long long> total;  // {suffix ids cut off, records}
     const uint64_t nt = (W + kCandTile - 1) / kCandTile;
     const bool scan = nt > kCandFewTiles;
+    const uint64_t stride = tile_stride(nt);
     GARY_TRY(total.alloc(2, s));
     GARY_CUDA(cudaMemsetAsync(total.p, 0, 16, s));
     GARY_TRY(tiles.alloc(std::max<uint64_t>(nt, 1), s));
@@ -421,7 +440,7 @@ int build_in_index(gary_graph *g, cudaStream_t s, const DevBuf<uint32_t> &len, I
     GARY_TRY(padded_rowid(g->dag, rowid, s));
     const unsigned grid = grid_for(nt * kThreads);
     if (W)
-      k_in_mark<<<grid, kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, len.p, marks.p, tiles.p, total.p);
+      k_in_mark<<<grid, kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, stride, len.p, marks.p, tiles.p, total.p);
     GARY_CUDA(cudaGetLastError());
     if (scan) thrust::exclusive_scan(pol, tiles.p, tiles.p + nt, tiles.p, (uint64_t)0);
     unsigned long long h[2] = {0, 0};
@@ -432,7 +451,7 @@ int build_in_index(gary_graph *g, cudaStream_t s, const DevBuf<uint32_t> &len, I
     GARY_TRY(keys.alloc(std::max<uint64_t>(m, 1), s));
     GARY_TRY(vals.alloc(std::max<uint64_t>(m, 1), s));
     if (m)
-      k_in_candidates<<<grid, kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, len.p, marks.p, tiles.p, scan,
+      k_in_candidates<<<grid, kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, stride, len.p, marks.p, tiles.p, scan,
                                                 keys.p, vals.p);
     GARY_CUDA(cudaGetLastError());
   }

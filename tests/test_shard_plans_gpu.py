@@ -41,19 +41,18 @@ def test_shards_of_separate_triangle_plans_add_up(cuda, scale, ef, tune):
         lib.gary_tune(b"reset", 0)
 
 
-def test_shards_of_plans_with_many_record_tiles(cuda):
-    """Lists of more than 2^14 tiles of 2048 padded words (one octet a vertex at
-    least), a skewed core among them."""
+@pytest.mark.parametrize("n,tiles", [(5_000_000, 1 << 14), (17_500_000, 1 << 16)])
+def test_shards_of_plans_with_many_record_tiles(cuda, n, tiles):
+    """Lists of more than 2^14 and more than 2^16 tiles of 2048 padded words: a
+    ring (one octet a vertex) with a skewed core."""
     import numpy as np
 
-    n = 5_000_000
-    rng = np.random.default_rng(14)
     s, d = gb.gen_rmat(16, 3, 1 << 20)
-    src = np.concatenate([s, rng.integers(0, n, 3 * n, dtype=np.uint32)])
-    dst = np.concatenate([d, rng.integers(0, n, 3 * n, dtype=np.uint32)])
+    ring = np.arange(n, dtype=np.uint32)
+    src, dst = np.concatenate([s, ring]), np.concatenate([d, np.roll(ring, 1)])
     ptr, idx = gb.csr_from_edges(src, dst, n)
     optr, oidx = O.orient(ptr, idx)
-    assert int(((np.diff(optr.astype(np.int64)) + 7) // 8).sum()) * 8 > 2048 << 14
+    assert int(((np.diff(optr.astype(np.int64)) + 7) // 8).sum()) * 8 > 2048 * tiles
     want = O.tri_count(optr, oidx)
     total = 0
     for k in range(3):
