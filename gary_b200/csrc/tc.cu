@@ -32,6 +32,7 @@
 #include <thrust/reduce.h>
 #include <thrust/scan.h>
 #include <thrust/transform.h>
+#include <thrust/transform_reduce.h>
 
 #include <algorithm>
 #include <memory>
@@ -240,7 +241,8 @@ __global__ void k_in_work(const uint32_t *__restrict__ keys, const uint2 *__rest
 }
 
 // pcost (optional): predicted cycles of a warp-class vertex, with tile target
-// tw_pred in the same unit; without it, costs are probe counts.
+// tw_pred in the same unit; without it, costs are probe counts.  tw_pred cycles
+// stand for warp_tile_cost probes.
 __global__ void k_classify(const uint2 *__restrict__ row, const uint32_t *__restrict__ adj,
                            const uint64_t *__restrict__ work,
                            const uint64_t *__restrict__ inptr, uint32_t n, PlanParams pp,
@@ -268,15 +270,17 @@ __global__ void k_classify(const uint2 *__restrict__ row, const uint32_t *__rest
       const uint64_t cp = dv <= kTinyOut ? work[v] + 8 * nin + 16 : work[v] + build + pp.vertex_overhead;
       // learned: predicted cycles, but never below the probe cost scaled to
       // the same tile target, so that no tile outgrows a plain one (a vertex
-      // the model under-rates would otherwise end the launch alone)
-      const uint64_t c = pred ? max(pcost[v] + 1, cp * tw_pred / pp.warp_tile_cost) : cp;
+      // the model under-rates would otherwise end the launch alone).  The model
+      // knows tiny vertices with a set only: theirs is the scaled probe cost.
+      auto scaled = [&](uint64_t probes) { return pred ? probes * tw_pred / pp.warp_tile_cost : probes; };
+      const uint64_t c = pred && dv > kTinyOut ? max(pcost[v] + 1, scaled(cp)) : max(scaled(cp), (uint64_t)1);
       const uint64_t tw = pred ? tw_pred : pp.warp_tile_cost;
       if (!warp_fits) {
         cls = kClassCta;
         kc = (uint32_t)min_u64((c + pp.cta_tile_cost - 1) / pp.cta_tile_cost, nin);
       } else if (c > tw) {
         cls = kClassSplit;
-        const uint64_t piece = max(tw, pp.split_floor * dv);  // every piece builds the set again
+        const uint64_t piece = max(tw, scaled(pp.split_floor * dv));  // every piece builds the set again
         kw = (uint32_t)min_u64((c + piece - 1) / piece, nin);
       } else {
         cls = kClassLight;
@@ -319,6 +323,13 @@ struct GroupTarget {
 struct IsLight {
   const uint8_t *vclass;
   __host__ __device__ bool operator()(uint32_t v) const { return vclass[v] == kClassLight; }
+};
+
+// Predicted cycles of a vertex that is counted with a set.
+struct SetCycles {
+  const uint2 *row;
+  const uint64_t *pcost;
+  __host__ __device__ uint64_t operator()(uint32_t v) const { return row[v].y > kTinyOut ? pcost[v] : 0u; }
 };
 
 struct LightCost {
@@ -562,7 +573,9 @@ int k3_plan(gary_graph *g, const PlanParams &pp_in, cudaStream_t s, gary_count_p
                                                 plan->in.inptr.p, n, pp.warp_cap, x.p, legal.p);
     k_predict<<<grid_for(n), 128, 0, s>>>(dmodel.p, x.p, legal.p, n, plan->variant.p, pcost.p);
     GARY_CUDA(cudaGetLastError());
-    const uint64_t total = thrust::reduce(pol, pcost.p, pcost.p + n, 0ull);
+    const uint64_t total = thrust::transform_reduce(pol, thrust::counting_iterator<uint32_t>(0),
+                                                    thrust::counting_iterator<uint32_t>(n),
+                                                    SetCycles{g->dag.row.p, pcost.p}, (uint64_t)0, thrust::plus<uint64_t>());
     // about 32 warp tiles per resident warp, in predicted cycles
     const uint64_t slots = (uint64_t)sm_count() * pp.min_blocks * tc_warps(pp.min_blocks) * 32;
     tw = std::max<uint64_t>(total / std::max<uint64_t>(slots, 1), 4096);
