@@ -361,6 +361,19 @@ int plan_slot(int pattern, int sched) { return (pattern - 3) * 2 + sched; }
 constexpr int kShardSlot = 2;    // + sched: a shard's plan where the whole count's had no room for rows
 constexpr int kProfileSlot = 7;  // the plan of gary_tc_features and gary_tc_profile: no hub rows
 
+// That plan: the counting plan where it has no hub rows, else one of its own.
+int profile_plan(gary_graph *g, cudaStream_t s, gary_count_plan **out) {
+  gary_count_plan *count = g->plans[plan_slot(GARY_PATTERN_TRIANGLE, GARY_SCHED_PLAIN)];
+  if (count && !count->hub.n_list) {
+    *out = count;
+    return GARY_OK;
+  }
+  if (!g->plans[kProfileSlot])
+    GARY_TRY(build_k3_plan(g, tuned_params(), s, &g->plans[kProfileSlot], nullptr, Rows::kNone));
+  *out = g->plans[kProfileSlot];
+  return GARY_OK;
+}
+
 PlanParams g_tuning;  // process-wide knobs of the counting plans (gary_tune)
 std::mutex g_tuning_mu;
 std::vector<float> g_model;  // process-wide cost model (gary_set_cost_model)
@@ -485,9 +498,9 @@ extern "C" int gary_tc_features(gary_graph *g, float *d_x, uint8_t *d_legal, voi
   GARY_CHECK_ARG(g && d_x && d_legal, "NULL argument");
   return guarded("gary_tc_features", [&] {
     cudaStream_t s = gary::as_stream(stream);
-    const int slot = gary::kProfileSlot;
-    if (!g->plans[slot]) GARY_TRY(gary::build_k3_plan(g, gary::tuned_params(), s, &g->plans[slot], nullptr, gary::Rows::kNone));
-    return gary::k3_features(g, g->plans[slot], d_x, d_legal, s);
+    gary_count_plan *plan = nullptr;
+    GARY_TRY(gary::profile_plan(g, s, &plan));
+    return gary::k3_features(g, plan, d_x, d_legal, s);
   });
 }
 
@@ -497,15 +510,15 @@ extern "C" int gary_tc_profile(gary_graph *g, int variant, uint64_t *d_cycles, u
   GARY_CHECK_ARG(variant >= -1 && variant <= 3, "variant must be -1 (plain) or 0..3");
   return guarded("gary_tc_profile", [&] {
     cudaStream_t s = gary::as_stream(stream);
-    const int slot = gary::kProfileSlot;
-    if (!g->plans[slot]) GARY_TRY(gary::build_k3_plan(g, gary::tuned_params(), s, &g->plans[slot], nullptr, gary::Rows::kNone));
+    gary_count_plan *plan = nullptr;
+    GARY_TRY(gary::profile_plan(g, s, &plan));
     gary::DevBuf<uint8_t> forced;
     if (variant >= 0) {
       GARY_TRY(forced.alloc(g->n, s));
       GARY_CUDA(cudaMemsetAsync(forced.p, variant, g->n, s));
     }
     GARY_CUDA(cudaMemsetAsync(d_cycles, 0, (uint64_t)g->n * 8, s));
-    return gary::launch_k3_ctl(g, g->plans[slot], reinterpret_cast<unsigned long long *>(d_count), s,
+    return gary::launch_k3_ctl(g, plan, reinterpret_cast<unsigned long long *>(d_count), s,
                                0, 1, variant >= 0 ? forced.p : nullptr,
                                reinterpret_cast<unsigned long long *>(d_cycles));
   });
