@@ -1345,12 +1345,14 @@ int build_coo(PaddedCSR &c, cudaStream_t s) {
               (unsigned long long)got, (unsigned long long)c.m);
     return GARY_ERR_CUDA;
   }
-  GARY_TRY(c.coo_row.alloc_persistent(c.m));
-  GARY_TRY(c.coo_col.alloc_persistent(c.m));
-  k_gather_pairs<<<grid_for(c.m), kThreads, 0, s>>>(words.p, c.m, rowid.p, c.adj.p, c.coo_row.p,
-                                                    c.coo_col.p);
+  DevBuf<uint32_t> row, col;  // the graph's once both are there
+  GARY_TRY(row.alloc_persistent(c.m));
+  GARY_TRY(col.alloc_persistent(c.m));
+  k_gather_pairs<<<grid_for(c.m), kThreads, 0, s>>>(words.p, c.m, rowid.p, c.adj.p, row.p, col.p);
   GARY_CUDA(cudaGetLastError());
   GARY_CUDA(cudaStreamSynchronize(s));
+  c.coo_row = std::move(row);
+  c.coo_col = std::move(col);
   return GARY_OK;
 }
 

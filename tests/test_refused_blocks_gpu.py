@@ -54,3 +54,20 @@ def test_counts_with_a_block_refused(cuda, skewed, pattern):
     # a plan that is refused a block is made again without rows: only blocks that
     # no plan can do without end a count, never all of them
     assert refused < BLOCKS // 2
+
+
+@pytest.mark.parametrize("k", [1, 2])
+def test_coo_view_with_a_block_refused(cuda, skewed, k):
+    """The COO view is refused its row or its column array: the next call builds both."""
+    ptr, idx, n, _ = skewed
+    with gb.Graph.upload(ptr, idx, n) as g:
+        _refuse(k)
+        try:
+            with pytest.raises(gb.GaryError):
+                g.device_coo()
+        finally:
+            _refuse(0)
+        coo = g.device_coo()
+        assert coo.rowIdx and coo.colIdx
+        p, i, _ = g.download()
+        assert int(p[-1]) == len(i) == len(idx) // 2
