@@ -490,7 +490,8 @@ def run_ours(args, dist):
             }
         work = stats.get("work") or 0
         roofline["probes"] = {"per_launch": work, "per_s": work / (ms_local / 1e3) if work else None,
-                              "definition": "ids of in-neighbour suffixes tested against a set of N+(v)"}
+                              "definition": "ids of in-neighbour suffixes covered: tested against a set of N+(v), or "
+                                            "counted by hub rows, many to an AND"}
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": dist.world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "strong",

@@ -118,8 +118,8 @@ int build_adj_rows(gary_graph *g, cudaStream_t s, AdjRows &adj);
 // middle-vertex walk still covers (all of it for a vertex not counted here).
 // Otherwise leaves hub.n_list 0 and len empty; hub.no_room says that they would
 // have paid.  (Required rows do not ask for room: a row of 512 bytes takes 57 ids
-// or more out of the walk, and each of them saves the plan 24 bytes of records to
-// sort.)
+// or more out of the walk, and each of them saves the plan 12 bytes to sort and 8
+// of index.)
 int build_hub_rows(gary_graph *g, cudaStream_t s, Rows use, HubRows &hub, DevBuf<uint32_t> &len);
 
 // The bits of word `word` (of a row) from bit position `from` on.

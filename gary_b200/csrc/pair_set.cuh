@@ -65,7 +65,7 @@ struct PairSet {
   }
 };
 
-// The warp's set of the d sorted ids at av (pair_log(d, last) = k > 0) in its
+// The warp's set of the d sorted ids at av (k = pair_log(d, n) > 0) in its
 // region tab.  False: an id found no place.  All 32 lanes call.
 __device__ __forceinline__ bool build_pair_set(const uint32_t *__restrict__ av, uint32_t d, int k, uint32_t *tab,
                                                int lane, PairSet &set) {

@@ -82,9 +82,9 @@ struct MinU64 {
 // Two passes, tile by tile of kCandTile words.  This one marks the words with a
 // record, a bit each, so that d+(v), a scattered read, is not read twice, and
 // counts them: tiles[q] of the q-th tile.  total[0] += the suffix ids past len[u],
-// total[1] += the records.  A first count, plan included, takes some 10 us more
-// than with one appending pass (RMAT-16 ef16 0.447 / 0.456 ms, RMAT-20 1.530 /
-// 1.540, RMAT-22 6.03 / 6.05).
+// total[1] += the records.  A first count, plan included, takes up to 15 us
+// more than with one appending pass (RMAT-16 ef16 0.446 / 0.450 ms, RMAT-20 1.521 /
+// 1.537, RMAT-22 6.03 / 6.05).
 constexpr int kCandPer = 8;
 constexpr uint32_t kCandTile = kThreads * kCandPer;
 constexpr int kCandWarps = kThreads / 32;
@@ -454,17 +454,19 @@ int build_in_index(gary_graph *g, cudaStream_t s, const DevBuf<uint32_t> &len, I
       k_in_mark<<<grid, kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, stride, len.p, marks.p, tiles.p, total.p);
     GARY_CUDA(cudaGetLastError());
     if (scan) thrust::exclusive_scan(pol, tiles.p, tiles.p + nt, tiles.p, (uint64_t)0);
+    // a word has one record at most: not waiting for their number here keeps the
+    // device busy over the allocations and the launch
+    GARY_TRY(keys.alloc(std::max<uint64_t>(W, 1), s));
+    GARY_TRY(vals.alloc(std::max<uint64_t>(W, 1), s));
+    if (W)
+      k_in_candidates<<<grid, kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, stride, len.p, marks.p, tiles.p, scan,
+                                                keys.p, vals.p);
+    GARY_CUDA(cudaGetLastError());
     unsigned long long h[2] = {0, 0};
     GARY_CUDA(cudaMemcpyAsync(h, total.p, 16, cudaMemcpyDeviceToHost, s));
     GARY_CUDA(cudaStreamSynchronize(s));
     in.hub_work = h[0];
     m = h[1];
-    GARY_TRY(keys.alloc(std::max<uint64_t>(m, 1), s));
-    GARY_TRY(vals.alloc(std::max<uint64_t>(m, 1), s));
-    if (m)
-      k_in_candidates<<<grid, kThreads, 0, s>>>(g->dag.row.p, g->dag.adj.p, rowid.p, W, stride, len.p, marks.p, tiles.p, scan,
-                                                keys.p, vals.p);
-    GARY_CUDA(cudaGetLastError());
   }
   if (m) {
     GARY_TRY(keys2.alloc(m, s));
@@ -658,8 +660,10 @@ constexpr uint32_t kWarpBitmapSpan = bitmap_max_span(kWarpTableSlots);  // ids a
 // 32-byte boundaries and are padded with kSentinel to a multiple of 8 words,
 // so an octet only ever holds words of its own list: ids up to and including
 // v before the suffix (all below min N+(v)) and padding (a suffix cut short by
-// hub rows ends with an octet).  Every set rejects
-// both as out of its [lo, lo + span] range, so no per-id mask is needed.
+// hub rows ends with an octet).  Every set rejects both, so no per-id mask is
+// needed: most as out of their [lo, lo + span] range, a pair set as ids that are
+// not in it (its entries and slots give an id back exactly, and padding has an
+// entry of more than 16 bits).
 // All 32 lanes must call.
 template <typename Set>
 __device__ __forceinline__ uint32_t probe_octet(const uint4 &a, const uint4 &b, const Set &set) {

@@ -69,7 +69,7 @@ struct PlanParams {
 };
 
 // The parameters a plan over `total_work` probes in `records` suffixes uses:
-// explicit values as given, the zeros resolved.
+// explicit values as given, the zeros resolved, split_floor always from the work.
 PlanParams resolve_params(PlanParams pp, uint64_t total_work, uint64_t records);
 
 // Process-wide tuning overrides (0 = keep the default), set by gary_tune().
@@ -108,7 +108,8 @@ enum : uint32_t { kPathBitmap = 0, kPathBuckets = 1, kPathStaged = 2, kPathSampl
 // In-edge index of the middle-vertex formulation.  For every oriented edge
 // u -> v whose list suffix after v is non-empty, and with d+(v) > 0:
 //   inedge[k] = {first word of N+(u) after v, length of that suffix}
-// (the suffix ends at u's first hub neighbour when u is counted by hub rows)
+// (where u is counted by hub rows, N+(u) ends for this with its ids below the hubs,
+// rounded up to whole octets)
 // grouped by v: v's records are inedge[inptr[v] .. inptr[v+1]).
 struct InIndex {
   DevBuf<uint2> inedge;

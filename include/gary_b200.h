@@ -78,7 +78,7 @@ typedef struct gary_graph_info {
   uint64_t wedges;           /* sum over (u,v) in E+ of d+(v) */
   uint64_t out_deg_sq;       /* sum over u of d+(u)^2 */
   uint64_t alg_bytes;        /* B_alg = sum over (u,v) in E+ of 4(d+(u)+d+(v)) + 24 */
-  uint64_t device_bytes;     /* bytes of device memory this graph holds */
+  uint64_t device_bytes;     /* bytes of the graph's own arrays; the plans of its counts come on top */
 } gary_graph_info;
 
 /* Raw views with the reference's field names (include/DeviceGraph.cuh:15-67).
@@ -168,8 +168,9 @@ int gary_count_shard_async(gary_graph *g, int pattern, int sched, uint32_t shard
  * shared-memory set that held N+(v) (bitmap of its id span, hash buckets,
  * the list staged whole by a bulk copy, evenly spaced samples for the
  * two-phase search), the launch's error word (0 when it ran clean), and the
- * triangle plan's work: the ids its kernel probes against a set, summed over
- * the whole plan (shards included).  For the triangle kernel also its makespan
+ * triangle plan's work: the suffix ids its kernel covers, probed against a set
+ * or counted by the bit rows of hubs, summed over the whole plan (shards
+ * included).  For the triangle kernel also its makespan
  * and the mean time at which its CTAs finished (device clock, from the first
  * CTA start): makespan / mean finish bounds what any other assignment of the
  * same tiles to CTAs could gain.  For benches and tests. */
@@ -235,12 +236,16 @@ int gary_gen_ba(uint32_t n, uint32_t m, uint64_t seed, uint32_t *src, uint32_t *
  * Process-wide parameters of the counting plans, applied to plans built after
  * the call (gary_graph_drop_plans discards a graph's cached plans):
  *   "warp_tile_cost"  target probes per warp tile; 0 (the default) sizes
- *                     it from the graph's work: about 32 tiles per resident
- *                     warp, between 2^11 and 2^15 probes
+ *                     it from the graph's work: about 128 tiles per resident
+ *                     warp, between 2^11 and 2^14 probes, and on graphs too
+ *                     small for that one tile per resident warp, of 128 probes
+ *                     at least.  A vertex is split into tiles of no less than
+ *                     16 probes (128 on graphs with 2^12 probes for every
+ *                     resident warp) per id of its list
  *   "cta_tile_cost"   target probes per CTA tile         (default 2^20)
  *   "vertex_overhead" fixed cost charged per vertex      (default 64)
  *   "min_blocks"      resident CTAs per SM, 2 or 3; 0 (the default) picks 3
- *                     from 2^31 probes on, else 2
+ *                     from 2^26 probes on, else 2
  *   "warp_cap"        largest out-degree d+(v) a warp's hash set takes
  *                     (8..512, default 512); larger lists whose id span is
  *                     too wide for a warp bitmap go to CTA tiles
